@@ -257,53 +257,53 @@ void launch_correct(const CorrArgs<T>& a, cudaStream_t s) {
 // staggered/func_global.h:875-890 with |S| of :823-870.  Collocated: per element
 // (lower-corner node index), collocated_AB3/func_global.h:342-384.
 // ---------------------------------------------------------------------------
+// One cell (element) per thread, one plane per blockIdx.z: the neighbours come through L1,
+// the wrapped column indices are computed once, and the model's wall factor is the plane's
+// constant SM.  96x96x64 FP64: 37.6 -> 15.5 us (19 MB of algorithmic traffic, L2-resident;
+// per-cell exp and pow in double and the index divisions bound the earlier form).
 template <typename T>
 struct GAcc {
     const T* v[3];
-    int ix, iy, iz, NX, NY;
+    size_t base;  // plane iz
+    int x[3], y[3];  // ix-1, ix, ix+1 and NX * (iy-1, iy, iy+1), wrapped
     size_t NXY;
+    __device__ __forceinline__ void init(const TurbArgs<T>& a, int ix, int iy, int iz) {
+        const Geom& g = a.g;
+        NXY = (size_t)g.NXY;
+        base = (size_t)iz * NXY;
+#pragma unroll
+        for (int c = 0; c < 3; c++) v[c] = a.v.c[c];
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            x[d] = wrapi(ix + d - 1, g.NX);
+            y[d] = wrapi(iy + d - 1, g.NY) * g.NX;
+        }
+    }
     __device__ __forceinline__ T operator()(int c, int dx, int dy, int dz) const {
-        const int x = wrapi(ix + dx, NX), y = wrapi(iy + dy, NY);
-        return __ldg(v[c] + (size_t)(iz + dz) * NXY + (size_t)y * NX + x);
+        return __ldg(v[c] + base + (long long)dz * (long long)NXY + (y[dy + 1] + x[dx + 1]));
     }
 };
 
 template <typename T>
-__device__ __forceinline__ T smag_nut(T AbsS, T dist, T vol, T inv_ls) {
-    const T yp = dist * inv_ls;
-    const T C_SMAG = T(0.1), C_exp = T(0.04 * 0.04 * 0.04);
-    const T fvd = 1 - exp(-C_exp * yp * yp * yp);
-    T Dl = C_SMAG * pow(vol, T(0.33333333333333333333));
-    if (Dl > T(0.41) * dist) Dl = T(0.41) * dist;
-    return fvd * Dl * Dl * AbsS;
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) k_turb_stag(TurbArgs<T> a) {
+__global__ void __launch_bounds__(KX* KY) k_turb_stag(TurbArgs<T> a) {
     const Geom& g = a.g;
-    const long long in = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (in >= g.N) return;
-    const int ix = (int)(in % g.NX), iy = (int)((in / g.NX) % g.NY), iz = (int)(in / g.NXY);
-    GAcc<T> A{{a.v.c[0], a.v.c[1], a.v.c[2]}, ix, iy, iz, g.NX, g.NY, (size_t)g.NXY};
+    const int ix = blockIdx.x * KX + threadIdx.x % KX, iy = blockIdx.y * KY + threadIdx.x / KX, iz = blockIdx.z;
+    if (ix >= g.NX || iy >= g.NY) return;
+    GAcc<T> A;
+    A.init(a, ix, iy, iz);
     StagZ<T> mz{iz, g.NZ, a.m.DZ, a.m.DZW, (T)g.hx, (T)g.hy, (T)g.inv_hx, (T)g.inv_hy, (T)g.visc, {}};
 #pragma unroll
     for (int k = 0; k < 6; k++) mz.pc[k] = a.m.PC[TC_PC * iz + k];
-    const T S = abs_strain(A, mz);
-    const T* ZZ = a.m.ZZ;
-    const T H = T(0.5) * (ZZ[g.NZ] - ZZ[0]);
-    const T Z = T(0.5) * (ZZ[iz] + ZZ[iz + 1]) - ZZ[0];
-    const T d = (Z < H) ? Z : 2 * H - Z;
-    a.nu_t[in] = smag_nut(S, d, (T)g.hx * (T)g.hy * a.m.DZ[iz], (T)g.inv_ls);
+    a.nu_t[A.base + (size_t)iy * g.NX + ix] = a.m.SM[iz] * abs_strain(A, mz);
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_turb_coll(TurbArgs<T> a) {
+__global__ void __launch_bounds__(KX* KY) k_turb_coll(TurbArgs<T> a) {
     const Geom& g = a.g;
-    const long long ie = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (ie >= g.N) return;
-    const int ix = (int)(ie % g.NX), iy = (int)((ie / g.NX) % g.NY), iz = (int)(ie / g.NXY);
-    if (iz >= g.NZ - 1) return;
-    GAcc<T> A{{a.v.c[0], a.v.c[1], a.v.c[2]}, ix, iy, iz, g.NX, g.NY, (size_t)g.NXY};
+    const int ix = blockIdx.x * KX + threadIdx.x % KX, iy = blockIdx.y * KY + threadIdx.x / KX, iz = blockIdx.z;
+    if (ix >= g.NX || iy >= g.NY) return;
+    GAcc<T> A;
+    A.init(a, ix, iy, iz);
     const T hz = (T)a.m.dDZ[iz];
     const T ihx = (T)g.inv_hx, ihy = (T)g.inv_hy;
     T gr[3][3];
@@ -320,19 +320,16 @@ __global__ void __launch_bounds__(256) k_turb_coll(TurbArgs<T> a) {
     gr[1][2] = T(0.5) * (gr[1][2] + gr[2][1]);
     T S = gr[0][0] * gr[0][0] + gr[1][1] * gr[1][1] + gr[2][2] * gr[2][2] +
           2 * (gr[0][1] * gr[0][1] + gr[0][2] * gr[0][2] + gr[1][2] * gr[1][2]);
-    S = sqrt(2 * S);
-    const double* ZZ = a.m.dZZ;
-    const T H = (T)(0.5 * (ZZ[g.NZ - 1] - ZZ[0]));
-    const T Z = (T)(0.5 * (ZZ[iz] + ZZ[iz + 1]));
-    const T d = (Z < H) ? Z : 2 * H - Z;
-    a.nu_t[ie] = smag_nut(S, d, (T)g.hx * (T)g.hy * hz, (T)g.inv_ls);
+    a.nu_t[A.base + (size_t)iy * g.NX + ix] = a.m.SM[iz] * sqrt(2 * S);
 }
 
 template <typename T>
 void launch_turb(const TurbArgs<T>& a, cudaStream_t s) {
-    const unsigned nb = (unsigned)((a.g.N + 255) / 256);
-    if (a.g.scheme == TC_SCHEME_COLLOC) k_turb_coll<T><<<nb, 256, 0, s>>>(a);
-    else k_turb_stag<T><<<nb, 256, 0, s>>>(a);
+    const bool coll = a.g.scheme == TC_SCHEME_COLLOC;
+    // collocated: the NZ-1 element layers between the node planes (the top plane keeps its value)
+    const dim3 grid((a.g.NX + KX - 1) / KX, (a.g.NY + KY - 1) / KY, coll ? a.g.NZ - 1 : a.g.NZ);
+    if (coll) k_turb_coll<T><<<grid, KX * KY, 0, s>>>(a);
+    else k_turb_stag<T><<<grid, KX * KY, 0, s>>>(a);
 }
 
 // ---------------------------------------------------------------------------

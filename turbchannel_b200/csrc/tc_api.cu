@@ -291,6 +291,7 @@ static MeshDev<T> mesh_dev(const tc_handle* h) {
     MeshDev<T> m;
     m.ZZ = t + 0 * L; m.DZ = t + 1 * L; m.DZW = t + 2 * L; m.GC1 = t + 3 * L; m.GC2 = t + 4 * L;
     m.GCZ = t + 5 * L; m.KERG = t + 6 * L; m.cellh = t + 7 * L; m.MAT_A = t + 8 * L; m.PC = t + 11 * L;
+    m.SM = t + (11 + TC_PC) * L;
     m.FK = h->fp64 ? nullptr : (const float*)h->fk;
     m.FK64 = h->fp64 ? (const double*)h->fk : nullptr;
     m.dZZ = d + 0 * L; m.dDZ = d + 1 * L; m.dDZW = d + 2 * L; m.dKERG = d + 6 * L; m.dcellh = d + 7 * L;
@@ -372,6 +373,25 @@ static void fill_plane_consts(const Geom& g, const HostMesh& hm, const T* t, T* 
         c[4] = T(-1) / (32 * (DZ[z] - C9 * DZW[z]) * hx * hy);
         c[5] = -T(1. / 32.) * ihx * ihy * GCZ[z];
         c[6] = c[7] = T(0);
+    }
+}
+
+// nu_t / |S| of the Smagorinsky-van Driest model per plane of cells (staggered/
+// func_global.h:875-890) or layer of elements (collocated_AB3/func_global.h:372-384):
+// f_vd min(0.1 vol^(1/3), 0.41 d)^2 with f_vd = 1 - exp(-(0.04 y+)^3).  It depends on z
+// only; evaluated per cell, its exp and pow took 30 of the kernel's 38 us at 96x96x64 FP64.
+static void fill_smagorinsky(const Geom& g, const HostMesh& hm, double* sm) {
+    const bool coll = g.scheme == TC_SCHEME_COLLOC;
+    const std::vector<double>& ZZ = hm.ZZ;
+    const int nl = coll ? g.NZ - 1 : g.NZ;
+    const double H = 0.5 * (ZZ[nl] - ZZ[0]);
+    for (int z = 0; z < nl; z++) {
+        const double zc = 0.5 * (ZZ[z] + ZZ[z + 1]) - (coll ? 0.0 : ZZ[0]);
+        const double d = zc < H ? zc : 2 * H - zc;
+        const double yp = d * g.inv_ls;
+        const double fvd = 1 - std::exp(-(0.04 * 0.04 * 0.04) * yp * yp * yp);
+        const double Dl = std::min(0.1 * std::pow(g.hx * g.hy * hm.DZ[z], 0.33333333333333333333), 0.41 * d);
+        sm[z] = fvd * Dl * Dl;
     }
 }
 
@@ -500,9 +520,9 @@ extern "C" int tc_create(const tc_params* prm, const double* zz, tc_handle** out
     TC_ALLOC(h->zfac, zfactor_bytes(g, (int)E));
     TC_ALLOC(h->zfac_low, zfactor_low_bytes(g));
     // mesh arrays, 9 slots of NZ+2 (the last one holds MAT_A, up to 3 NZ entries), then
-    // the per-plane reciprocals (TC_PC per plane)
+    // the per-plane reciprocals (TC_PC per plane) and the Smagorinsky factor (one per plane)
     const int L = g.NZ + 2;
-    const size_t mlen = (size_t)8 * L + 3 * (size_t)L + (size_t)TC_PC * L;
+    const size_t mlen = (size_t)8 * L + 3 * (size_t)L + (size_t)TC_PC * L + (size_t)L;
     TC_ALLOC(h->mesh_t, mlen * E);
     TC_ALLOC(h->mesh_d, mlen * sizeof(double));
     {
@@ -515,6 +535,7 @@ extern "C" int tc_create(const tc_params* prm, const double* zz, tc_handle** out
         put(6, hm.KERG); put(7, hm.cellh); put(8, hm.MAT_A);
         const size_t pc0 = (size_t)11 * L;
         fill_plane_consts<double>(g, hm, md.data(), md.data() + pc0);
+        fill_smagorinsky(g, hm, md.data() + pc0 + (size_t)TC_PC * L);
         if (cudaMemcpy(h->mesh_d, md.data(), mlen * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) {
             free_all(h); delete h;
             return fail(TC_E_CUDA, "tc_create: mesh upload failed");

@@ -39,6 +39,7 @@ constexpr int TC_FK = 48, TC_FK64 = 24;
 template <typename T>
 struct MeshDev {
     const T *ZZ, *DZ, *DZW, *GC1, *GC2, *GCZ, *KERG, *MAT_A, *cellh, *PC;
+    const T* SM = nullptr;  // Smagorinsky-van Driest: nu_t / |S| of each plane (staggered) or element layer (collocated)
     const float* FK = nullptr;
     const double* FK64 = nullptr;
     const double *dZZ, *dDZ, *dDZW, *dKERG, *dMAT_A, *dcellh;

@@ -183,10 +183,10 @@ template <typename T> int launch_div_xfft(const DivFftArgs<T>& a, cudaStream_t s
 template <typename T> void launch_yfft(const YFftArgs<T>& a, cudaStream_t s);
 template <typename T> void launch_zsolve(const ZSolveArgs<T>& a, cudaStream_t s, cudaStream_t side, cudaEvent_t fork,
                                        cudaEvent_t join);
-// factored solve (step path): launch_zfactor once at creation, then launch_zsolve_fac
+// factored solve (step path, k_zsolve.cu): launch_zfactor once at creation, then launch_zsolve_fac
 template <typename T> void launch_zfactor(const ZSolveArgs<T>& a, cudaStream_t s);
-template <typename T> void launch_zsolve_fac(const ZSolveArgs<T>& a, cudaStream_t s, cudaStream_t side,
-                                           cudaEvent_t fork, cudaEvent_t join);
+template <typename T> int launch_zsolve_fac(const ZSolveArgs<T>& a, cudaStream_t s, cudaStream_t side,
+                                           cudaEvent_t fork, cudaEvent_t join);  // returns launches
 template <typename T> void launch_ixfft(const IxFftArgs<T>& a, cudaStream_t s);
 // two-pass register FFT versions (k_fft.cu); false when the length has none
 template <typename T> int launch_div_xfft_reg(const DivFftArgs<T>& a, cudaStream_t s);  // 0: no such path

@@ -202,7 +202,7 @@ struct tc_handle {
     void* ptmp = nullptr;
     void* spec = nullptr;
     void* zfac = nullptr;  // time-independent factors of the z-matrices (k_zfactor)
-    void* zfac_low = nullptr;  // double factors of the low modes
+    void* zfac_low = nullptr;  // double factors of the low modes (mixed mode)
     void* mesh_t = nullptr;     // mesh arrays in T
     void* fk = nullptr;         // flux kernels' interior-plane constants (float pairs mixed, doubles FP64 VV4)
     double* mesh_d = nullptr;   // mesh arrays in double
@@ -518,7 +518,7 @@ extern "C" int tc_create(const tc_params* prm, const double* zz, tc_handle** out
     TC_ALLOC(h->ptmp, N * E);
     TC_ALLOC(h->spec, (size_t)g.NXH * g.NY * g.NZ * 2 * E);
     TC_ALLOC(h->zfac, zfactor_bytes(g, (int)E));
-    TC_ALLOC(h->zfac_low, zfactor_low_bytes(g));
+    if (!h->fp64) TC_ALLOC(h->zfac_low, zfactor_low_bytes(g));
     // mesh arrays, 9 slots of NZ+2 (the last one holds MAT_A, up to 3 NZ entries), then
     // the per-plane reciprocals (TC_PC per plane) and the Smagorinsky factor (one per plane)
     const int L = g.NZ + 2;
@@ -617,7 +617,7 @@ extern "C" int tc_create(const tc_params* prm, const double* zz, tc_handle** out
     }
     if (h->nu_t) cudaMemsetAsync(h->nu_t, 0, N * E, h->st);
     cudaMemsetAsync(h->zfac, 0, zfactor_bytes(g, (int)E), h->st);
-    cudaMemsetAsync(h->zfac_low, 0, zfactor_low_bytes(g), h->st);
+    if (h->zfac_low) cudaMemsetAsync(h->zfac_low, 0, zfactor_low_bytes(g), h->st);
     if (h->fp64) {
         ZSolveArgs<double> za{g, mesh_dev<double>(h), mode_tabs(h), (cplx<double>*)h->spec, nullptr, h->err_flag, h->zfac,
                               h->zfac_low};
@@ -849,7 +849,7 @@ static void poisson(tc_handle* h, const void* rhs_vec, const void* rhs_scalar, v
     if (!pf) launch_yfft<T>(ya, h->st);
     if (mk) mark(h, 4, eb);
     ZSolveArgs<T> za{g, mesh_dev<T>(h), mode_tabs(h), (cplx<T>*)h->spec, nullptr, h->err_flag, h->zfac, h->zfac_low};
-    launch_zsolve_fac<T>(za, h->st, h->side, h->ev_fork, h->ev_join);
+    const int nz = launch_zsolve_fac<T>(za, h->st, h->side, h->ev_fork, h->ev_join);
     if (mk) mark(h, 5, eb);
     ya.sign = +1;
     if (!plane) launch_yfft<T>(ya, h->st);
@@ -857,7 +857,7 @@ static void poisson(tc_handle* h, const void* rhs_vec, const void* rhs_scalar, v
     IxFftArgs<T> ia{g, (const cplx<T>*)h->spec, (T*)p_out, h->px, twx<T>(h), (T)(1.0 / ((double)g.NX * g.NY))};
     if (!(plane && launch_ixyfft_plane<T>(ia, twy<T>(h), h->st))) launch_ixfft<T>(ia, h->st);
     if (mk) mark(h, 7, eb);
-    h->launches += ndx + (pf ? 0 : 1) + 2 + (plane ? 1 : 2);
+    h->launches += ndx + (pf ? 0 : 1) + nz + (plane ? 1 : 2);
 }
 
 template <typename T>
@@ -1476,6 +1476,35 @@ static int srk_step_impl(tc_handle* h, double tau) {
     return check_launch("tc_srk_step");
 }
 
+static void run_graph_drop(tc_handle* h);
+
+// The mixed SRK step solves its banded systems from factors of its own layout: rebuilt once,
+// when the handle becomes an SRK one.
+static int srk_refactor(tc_handle* h) {
+    TC_CUDA(cudaStreamSynchronize(h->st));
+    run_graph_drop(h);  // a captured run holds the old factors
+    const Geom& g = h->g;
+    const size_t nf = zfactor_bytes(g, (int)h->esz), nl = zfactor_low_bytes(g);
+    void *f = nullptr, *fl = nullptr;
+    if (cudaMalloc(&f, nf) != cudaSuccess || cudaMalloc(&fl, nl) != cudaSuccess) {
+        cudaGetLastError();
+        if (f) cudaFree(f);
+        h->srk.S = 0;
+        h->g.norm_srk = 0;  // the handle keeps its factors
+        return fail(TC_E_NOMEM, "tc_srk_init: z-solve factors");
+    }
+    cudaFree(h->zfac);
+    cudaFree(h->zfac_low);
+    h->zfac = f;
+    h->zfac_low = fl;
+    TC_CUDA(cudaMemsetAsync(f, 0, nf, h->st));
+    TC_CUDA(cudaMemsetAsync(fl, 0, nl, h->st));
+    ZSolveArgs<float> za{g, mesh_dev<float>(h), mode_tabs(h), (cplx<float>*)h->spec, nullptr, h->err_flag, h->zfac,
+                         h->zfac_low};
+    launch_zfactor<float>(za, h->st);
+    return check_launch("tc_srk_init");
+}
+
 extern "C" int tc_srk_init(tc_handle* h, int imex_type, int nstages, const double* butcher_e, const double* butcher_i,
                            int stab_type, double alpha_tau) {
     if (!h || !butcher_e || !butcher_i) return fail(TC_E_ARG, "tc_srk_init: null argument");
@@ -1515,8 +1544,9 @@ extern "C" int tc_srk_init(tc_handle* h, int imex_type, int nstages, const doubl
         s.d[j] = 0.;
         for (int k = 0; k < j; k++) s.d[j] -= s.BI[j * S + k] * s.d[k] / a_ss;
     }
+    const bool refactor = !h->fp64 && !h->g.norm_srk;
     h->g.norm_srk = 1;  // the SRK pressure normalisation (collocated_SRK/func_global.h:130-137)
-    return TC_OK;
+    return refactor ? srk_refactor(h) : TC_OK;
 }
 
 extern "C" int tc_srk_step(tc_handle* h, double t, double tau) {

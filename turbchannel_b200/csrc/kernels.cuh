@@ -222,10 +222,11 @@ template <typename T> void launch_turb_mlp(const TurbArgs<T>& a, const float* P,
 template <typename T> void launch_flux_mlp(const FluxArgs<T>& a, const float* P, T* nu_out, cudaStream_t s);
 void launch_mlp_grad(const float* P, const float* X, const float* Y, long long n, float* part, float* grad,
                      cudaStream_t s);
-void launch_mlp_adam(float* P, float* M, float* V, const float* grad, float lr, int step, cudaStream_t s);
+// one training batch: gradient, Adam update, *loss += the batch's loss sum
+void launch_mlp_step(float* P, float* M, float* V, const float* X, const float* Y, long long n, float* part, float* loss,
+                     float lr, int step, cudaStream_t s);
 void launch_mlp_forward(const float* P, const float* X, long long n, float* out, cudaStream_t s);
 int mlp_grad_blocks(long long n);
-void launch_mlp_loss_acc(float* acc, const float* grad, cudaStream_t s);  // acc += loss sum in grad
 
 size_t zsolve_scratch_bytes(const Geom& g, int elem_bytes);
 size_t zfactor_bytes(const Geom& g, int elem_bytes);

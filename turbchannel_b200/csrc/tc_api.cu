@@ -1897,9 +1897,8 @@ extern "C" int tc_mlp_train(tc_mlp* m, int epochs, long long batch, float lr, fl
     for (int e = 0; e < epochs; e++) {
         for (long long off = 0; off < m->n; off += bsz) {
             const long long nb = std::min(bsz, m->n - off);
-            launch_mlp_grad(m->P, m->X + off * MLP_IN, m->Y + off, nb, m->part, m->grad, m->st);
-            launch_mlp_loss_acc(m->loss + e, m->grad, m->st);
-            launch_mlp_adam(m->P, m->M, m->V, m->grad, lr, ++m->step, m->st);
+            launch_mlp_step(m->P, m->M, m->V, m->X + off * MLP_IN, m->Y + off, nb, m->part, m->loss + e, lr, ++m->step,
+                            m->st);
         }
     }
     if ((rc = check_launch("tc_mlp_train"))) return rc;

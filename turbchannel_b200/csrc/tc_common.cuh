@@ -92,6 +92,31 @@ __host__ __device__ __forceinline__ cplx<T> cmul(cplx<T> a, cplx<T> b) {
 }
 
 // ---------------------------------------------------------------------------
+// Programmatic dependent launch: a kernel launched with launch_pdl may start while the
+// kernel before it in its stream still runs; pdl_wait returns once that kernel (and so all
+// before it, each of them waiting first) has completed and its writes are visible.  Only
+// constants and data no kernel writes may be touched before it.  pdl_launch lets the next
+// kernel start its own prologue.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
+template <typename... P, typename... A>
+static inline void launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, kern, P(args)...);
+}
+
+// ---------------------------------------------------------------------------
 // Async global->shared copies (LDGSTS).  Sizes 4, 8 or 16 bytes.
 // ---------------------------------------------------------------------------
 template <int BYTES>

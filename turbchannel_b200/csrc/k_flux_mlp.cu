@@ -96,9 +96,9 @@ struct MCopy {
 // nu_t of plane zc over the tile and its one-cell halo, into the nu_t ring slot zc % 3;
 // the tile's own cells also to the nu_t array.  Every warp takes batches of 32 cells:
 // each lane forms its cell's features (the centred-velocity gradient of k_turb_mlp,
-// differences in T, then float), then two 16-row tiles go through the network.
+// differences in T, then float), then the 32 samples go through the network.
 template <typename T, int H>
-__device__ __forceinline__ void nut_plane(const Geom& g, const double* ZZ, const T* ring, T* nts, float (*Xs)[MLP_IN],
+__device__ __forceinline__ void nut_plane(const Geom& g, const MeshDev<T>& m, const T* ring, T* nts, __nv_bfloat16 (*Xs)[8],
                                           const MlpSmem& S, int zc, int x0, int y0, T* nu_out) {
     using R = MRing<T, H>;
     const int NX = g.NX, NY = g.NY, NZ = g.NZ;
@@ -107,11 +107,7 @@ __device__ __forceinline__ void nut_plane(const Geom& g, const double* ZZ, const
     const float sc = (float)(nu / (utau * utau));
     const float gx = (float)(0.25 * g.inv_hx), gy = (float)(0.25 * g.inv_hy);
     const bool lo = zc > 0, hi = zc + 1 < NZ, hi2 = zc + 2 < NZ;
-    const double zm = lo ? 0.5 * (ZZ[zc - 1] + ZZ[zc]) : ZZ[0];
-    const double zp = hi ? 0.5 * (ZZ[zc + 1] + ZZ[zc + 2]) : ZZ[NZ];
-    const float gz = (float)(0.5 / (zp - zm));
-    const double zcc = 0.5 * (ZZ[zc] + ZZ[zc + 1]);
-    const float yplus = (float)(fmin(zcc - ZZ[0], ZZ[NZ] - zcc) * utau / nu);
+    const float gz = (float)m.LGZ[zc], yp = (float)m.LYP[zc];
     // plane pointers of component c at z-offset dz (planes outside the channel are never read)
     auto P = [&](int c, int dz) -> const T* { return ring + R::slot(zc + dz) * 3 * R::PL + c * R::PL; };
     const T *u0 = P(0, 0), *v0 = P(1, 0), *w0 = P(2, 0);
@@ -140,34 +136,20 @@ __device__ __forceinline__ void nut_plane(const Geom& g, const double* ZZ, const
             G[0][2] = (float)(uzp - uzm) * gz;
             G[1][2] = (float)(vzp - vzm) * gz;
             G[2][2] = (float)(wzp - wzm) * gz;
-            les_features_f(G, sc, yplus, Xs[32 * wid + lane]);
+            les_features_bf16(G, sc, yp, Xs[32 * wid + lane]);
+        } else {
+            *reinterpret_cast<uint4*>(Xs[32 * wid + lane]) = make_uint4(0u, 0u, 0u, 0u);
         }
         __syncwarp();
-#pragma unroll 1
-        for (int hh = 0; hh < 2; hh++) {
-            const int nr = min(16, NRC - (32 * b + 16 * hh));
-            if (nr <= 0) break;
-            unsigned ax[4];
-            feature_fragment(&Xs[32 * wid + 16 * hh][0], MLP_IN, nr, ax);
-            Acc64 z1, z2;
-            unsigned h1a[4][4];
-            float z3[2];
-            mlp_forward_tile(S, ax, z1, z2, h1a, z3);
-            if (t == 0) {
-#pragma unroll
-                for (int k = 0; k < 2; k++) {
-                    const int row = gq + 8 * k;
-                    if (row < nr) {
-                        const int rr = 32 * b + 16 * hh + row;
-                        const T val = (T)(nu * softplus(z3[k]));
-                        nslot[rr] = val;
-                        const int X = rr % NRX - 1, Y = rr / NRX - 1;
-                        const int ix = x0 + X, iy = y0 + Y;
-                        if (X >= 0 && X < FMX && Y >= 0 && Y < FMY && ix < NX && iy < NY)
-                            nu_out[(size_t)zc * NX * NY + (size_t)iy * NX + ix] = val;
-                    }
-                }
-            }
+        const float z3 = mlp_infer32(S, &Xs[32 * wid]);
+        const int rr = 32 * b + 16 * (t >> 1) + 8 * (t & 1) + gq;
+        if (rr < NRC) {
+            const T val = (T)(nu * softplus(z3));
+            nslot[rr] = val;
+            const int X = rr % NRX - 1, Y = rr / NRX - 1;
+            const int ix = x0 + X, iy = y0 + Y;
+            if (X >= 0 && X < FMX && Y >= 0 && Y < FMY && ix < NX && iy < NY)
+                nu_out[(size_t)zc * NX * NY + (size_t)iy * NX + ix] = val;
         }
         __syncwarp();
     }
@@ -182,7 +164,7 @@ __global__ void __launch_bounds__(FMX* FMY, 1) k_flux_mlp(FluxArgs<T> a, const f
     extern __shared__ __align__(16) unsigned char smraw[];
     T* ring = reinterpret_cast<T*>(smraw);
     T* nts = ring + R::RS * 3 * R::PL;                                   // [3][NRC]
-    float(*Xs)[MLP_IN] = reinterpret_cast<float(*)[MLP_IN]>(nts + 3 * NRC);  // [8 warps x 32][6]
+    __nv_bfloat16(*Xs)[8] = reinterpret_cast<__nv_bfloat16(*)[8]>(nts + 3 * NRC);  // [8 warps x 32][8]
     __shared__ MlpSmem S;
     __shared__ double sbuf[32];
     mlp_load_smem(S, P);
@@ -196,7 +178,6 @@ __global__ void __launch_bounds__(FMX* FMY, 1) k_flux_mlp(FluxArgs<T> a, const f
     const int ix = x0 + tx, iy = y0 + ty;
     const bool own = ix < NX && iy < NY;
     const int zlo = SCHEME == TC_SCHEME_VV4 ? 3 : 1, zhi = SCHEME == TC_SCHEME_VV4 ? NZ - 4 : NZ - 2;
-    const double* ZZ = a.m.dZZ;
 
     MCopy<T, H, VEC> cp;
     cp.init(x0, y0, NX, NY, g.N);
@@ -205,8 +186,8 @@ __global__ void __launch_bounds__(FMX* FMY, 1) k_flux_mlp(FluxArgs<T> a, const f
     cp_async_commit();
     cp_async_wait<0>();
     __syncthreads();  // also publishes the network's shared-memory image
-    if (zb - 1 >= 0) nut_plane<T, H>(g, ZZ, ring, nts, Xs, S, zb - 1, x0, y0, nu_out);
-    nut_plane<T, H>(g, ZZ, ring, nts, Xs, S, zb, x0, y0, nu_out);
+    if (zb - 1 >= 0) nut_plane<T, H>(g, a.m, ring, nts, Xs, S, zb - 1, x0, y0, nu_out);
+    nut_plane<T, H>(g, a.m, ring, nts, Xs, S, zb, x0, y0, nu_out);
     __syncthreads();  // the ring slot of plane zb - 2 is refilled by the first iteration
 
     StagZ<T> mz;
@@ -239,7 +220,7 @@ __global__ void __launch_bounds__(FMX* FMY, 1) k_flux_mlp(FluxArgs<T> a, const f
         }
         cp_async_wait<1>();
         __syncthreads();  // plane z+3 staged; nu_t slot (z+1) % 3 free (plane z-2 done)
-        if (z + 1 < NZ) nut_plane<T, H>(g, ZZ, ring, nts, Xs, S, z + 1, x0, y0, nu_out);
+        if (z + 1 < NZ) nut_plane<T, H>(g, a.m, ring, nts, Xs, S, z + 1, x0, y0, nu_out);
         __syncthreads();
         mz.iz = z;
 #pragma unroll
@@ -292,7 +273,7 @@ __global__ void __launch_bounds__(FMX* FMY, 1) k_flux_mlp(FluxArgs<T> a, const f
 template <typename T, int SCHEME>
 static size_t flux_mlp_smem() {
     using R = MRing<T, SCHEME == TC_SCHEME_VV4 ? 3 : 1>;
-    return sizeof(T) * ((size_t)R::RS * 3 * R::PL + 3 * NRC) + sizeof(float) * FMX * FMY * MLP_IN;
+    return sizeof(T) * ((size_t)R::RS * 3 * R::PL + 3 * NRC) + sizeof(__nv_bfloat16) * FMX * FMY * 8;
 }
 
 template <typename T, int SCHEME, int ORDER>

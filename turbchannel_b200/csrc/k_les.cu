@@ -166,119 +166,90 @@ __global__ void __launch_bounds__(256) k_les_features(const float* __restrict__ 
 
 // nu_t of a run from the learned closure.  P: packed FP32 parameters.  Each warp takes
 // 32 cells at a time: every lane gathers its cell's velocity gradient (differences in
-// T, then float) and features, then two 16-row tiles go through the network on the
-// tensor cores.  Staggered (COLL = false): the centred-velocity gradient of the cell.
-// Collocated (COLL = true): the elements between 8 nodes, where that scheme keeps nu_t
-// (iz < NZ-1, the top plane untouched as in the Smagorinsky kernel), with the element
-// gradient of the nodal velocity -- the network's inputs are invariants of the resolved
-// gradient in wall units and y+, the same physical quantities for both schemes.
+// T, then float) and its features, then the network runs on the 32 samples at once
+// (mlp_infer32) and every lane finishes one of them.  Staggered (COLL = false): the
+// centred-velocity gradient of the cell.  Collocated (COLL = true): the elements between 8
+// nodes, where that scheme keeps nu_t (iz < NZ-1, the top plane untouched as in the
+// Smagorinsky kernel), with the element gradient of the nodal velocity -- the network's
+// inputs are invariants of the resolved gradient in wall units and y+, the same physical
+// quantities for both schemes.
+// Bound by instruction issue and the special-function unit: 128 SiLU per cell at 1.5
+// operations each are 24 us of that unit at 96x96x64 mixed, where the kernel takes 58 us (106 with
+// 16-sample tiles, two operations per SiLU, 64-bit index divisions and the full 3 x 3 products).
 template <typename T, bool COLL>
 __global__ void __launch_bounds__(128, 4) k_turb_mlp(TurbArgs<T> a, const float* __restrict__ P) {
     __shared__ MlpSmem S;
-    __shared__ float Xs[4][32][MLP_IN];
+    __shared__ __align__(16) __nv_bfloat16 Xb[4][32][8];
     mlp_load_smem(S, P);
     __syncthreads();
     const Geom& g = a.g;
     const int NX = g.NX, NY = g.NY, NZ = g.NZ;
-    const size_t NXY = (size_t)NX * NY;
+    const unsigned NXY = (unsigned)g.NXY, N = (unsigned)g.N;  // 3 N < 2^32 (checked at creation)
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, gq = lane >> 2, t = lane & 3;
-    const double nu = g.visc, utau = g.inv_ls * g.visc;
-    const float sc = (float)(nu / (utau * utau));
+    const double utau = g.inv_ls * g.visc;
+    const float sc = (float)(g.visc / (utau * utau));
     const float gx = (float)(0.25 * g.inv_hx), gy = (float)(0.25 * g.inv_hy);
-    const T* __restrict__ u = a.v.c[0];
-    const T* __restrict__ v = a.v.c[1];
-    const T* __restrict__ w = a.v.c[2];
-    const double* ZZ = a.m.dZZ;
-    const long long N = g.N, ngrp = (N + 31) / 32;
-    for (long long grp = (long long)blockIdx.x * 4 + wid; grp < ngrp; grp += (long long)gridDim.x * 4) {
-        const long long c0 = grp * 32;
-        const int nrow = (int)min(32LL, N - c0);
-        if (COLL && lane < nrow && (c0 + lane) / (long long)NXY >= NZ - 1) {
-#pragma unroll
-            for (int k = 0; k < MLP_IN; k++) Xs[wid][lane][k] = 0.f;  // top node plane: no element
-        } else if (COLL && lane < nrow) {
-            const long long c = c0 + lane;
-            const int ix = (int)(c % NX), iy = (int)((c / NX) % NY), iz = (int)(c / NXY);
-            const int xp = ix + 1 == NX ? 0 : ix + 1, yp = iy + 1 == NY ? 0 : iy + 1;
-            const size_t p0 = (size_t)iz * NXY, p1 = p0 + NXY;
-            const size_t i00 = (size_t)iy * NX + ix, i10 = (size_t)iy * NX + xp, i01 = (size_t)yp * NX + ix,
-                         i11 = (size_t)yp * NX + xp;
-            const float ghx = (float)(0.25 * g.inv_hx), ghy = (float)(0.25 * g.inv_hy);
-            const float ghz = (float)(0.25 / (a.m.dZZ[iz + 1] - a.m.dZZ[iz]));
+    const unsigned top = COLL ? N - NXY : N;  // first cell without element
+    const unsigned ngrp = (N + 31u) / 32u;
+    for (unsigned grp = blockIdx.x * 4 + wid; grp < ngrp; grp += gridDim.x * 4) {
+        const unsigned c0 = grp * 32u, c = c0 + lane;
+        if (c < top) {
+            const unsigned iz = c / NXY, r = c - iz * NXY, iy = r / (unsigned)NX, ix = r - iy * (unsigned)NX;
+            const unsigned xp = (int)ix + 1 == NX ? 0u : ix + 1u, yp = (int)iy + 1 == NY ? 0u : iy + 1u;
+            const float gz = (float)a.m.LGZ[iz];
             float G[3][3];
+            if constexpr (COLL) {
+                const unsigned p0 = iz * NXY, p1 = p0 + NXY;
+                const unsigned i00 = iy * NX + ix, i10 = iy * NX + xp, i01 = yp * NX + ix, i11 = yp * NX + xp;
 #pragma unroll
-            for (int cc = 0; cc < 3; cc++) {
-                const T* q = a.v.c[cc];
-                const T q000 = q[p0 + i00], q100 = q[p0 + i10], q010 = q[p0 + i01], q110 = q[p0 + i11];
-                const T q001 = q[p1 + i00], q101 = q[p1 + i10], q011 = q[p1 + i01], q111 = q[p1 + i11];
-                G[cc][0] = (float)((q100 + q110 + q101 + q111) - (q000 + q010 + q001 + q011)) * ghx;
-                G[cc][1] = (float)((q010 + q110 + q011 + q111) - (q000 + q100 + q001 + q101)) * ghy;
-                G[cc][2] = (float)((q001 + q101 + q011 + q111) - (q000 + q100 + q010 + q110)) * ghz;
+                for (int cc = 0; cc < 3; cc++) {
+                    const T* __restrict__ q = a.v.c[cc];
+                    const T q000 = q[p0 + i00], q100 = q[p0 + i10], q010 = q[p0 + i01], q110 = q[p0 + i11];
+                    const T q001 = q[p1 + i00], q101 = q[p1 + i10], q011 = q[p1 + i01], q111 = q[p1 + i11];
+                    G[cc][0] = (float)((q100 + q110 + q101 + q111) - (q000 + q010 + q001 + q011)) * gx;
+                    G[cc][1] = (float)((q010 + q110 + q011 + q111) - (q000 + q100 + q001 + q101)) * gy;
+                    G[cc][2] = (float)((q001 + q101 + q011 + q111) - (q000 + q100 + q010 + q110)) * gz;
+                }
+            } else {
+                const T* __restrict__ u = a.v.c[0];
+                const T* __restrict__ v = a.v.c[1];
+                const T* __restrict__ w = a.v.c[2];
+                const unsigned xm = ix == 0 ? NX - 1u : ix - 1u, xpp = (int)xp + 1 == NX ? 0u : xp + 1u;
+                const unsigned ym = iy == 0 ? NY - 1u : iy - 1u, ypp = (int)yp + 1 == NY ? 0u : yp + 1u;
+                const unsigned pl = iz * NXY;
+                const unsigned r0 = pl + iy * NX, rm = pl + ym * NX, rp = pl + yp * NX, rpp = pl + ypp * NX;
+                const bool lo = iz > 0, hi = (int)iz + 1 < NZ;
+                // cell-centred values: u_c = (u_x + u_{x+1})/2, v_c = (v_y + v_{y+1})/2,
+                // w_c = (w_z + w_{z+1})/2 (w_NZ = 0); central differences, the wall value 0
+                // replacing a missing z-neighbour
+                G[0][0] = (float)((u[r0 + xpp] + u[r0 + xp]) - (u[r0 + ix] + u[r0 + xm])) * gx;
+                G[0][1] = (float)((u[rp + ix] + u[rp + xp]) - (u[rm + ix] + u[rm + xp])) * gy;
+                G[1][0] = (float)((v[r0 + xp] + v[rp + xp]) - (v[r0 + xm] + v[rp + xm])) * gx;
+                G[1][1] = (float)((v[rpp + ix] + v[rp + ix]) - (v[r0 + ix] + v[rm + ix])) * gy;
+                const T w0 = w[r0 + ix], w1 = hi ? w[r0 + ix + NXY] : T(0);
+                G[2][0] = (float)((w[r0 + xp] + (hi ? w[r0 + xp + NXY] : T(0))) -
+                                  (w[r0 + xm] + (hi ? w[r0 + xm + NXY] : T(0)))) * gx;
+                G[2][1] = (float)((w[rp + ix] + (hi ? w[rp + ix + NXY] : T(0))) -
+                                  (w[rm + ix] + (hi ? w[rm + ix + NXY] : T(0)))) * gy;
+                // z: (q(z+1) - q(z-1)) / (zc(z+1) - zc(z-1)) with zc the wall plane at a wall
+                const T uzp = hi ? u[r0 + ix + NXY] + u[r0 + xp + NXY] : T(0);
+                const T uzm = lo ? u[r0 + ix - NXY] + u[r0 + xp - NXY] : T(0);
+                const T vzp = hi ? v[r0 + ix + NXY] + v[rp + ix + NXY] : T(0);
+                const T vzm = lo ? v[r0 + ix - NXY] + v[rp + ix - NXY] : T(0);
+                const T wzp = hi ? w1 + ((int)iz + 2 < NZ ? w[r0 + ix + 2u * NXY] : T(0)) : T(0);
+                const T wzm = lo ? w[r0 + ix - NXY] + w0 : T(0);
+                G[0][2] = (float)(uzp - uzm) * gz;
+                G[1][2] = (float)(vzp - vzm) * gz;
+                G[2][2] = (float)(wzp - wzm) * gz;
             }
-            const double* ZZ = a.m.dZZ;
-            const double zc = 0.5 * (ZZ[iz] + ZZ[iz + 1]);
-            const double d = fmin(zc - ZZ[0], ZZ[NZ - 1] - zc);
-            les_features_f(G, sc, (float)(d * utau / nu), Xs[wid][lane]);
-        } else if (lane < nrow) {
-            const long long c = c0 + lane;
-            const int ix = (int)(c % NX), iy = (int)((c / NX) % NY), iz = (int)(c / NXY);
-            const int xm = ix == 0 ? NX - 1 : ix - 1, xp = ix + 1 == NX ? 0 : ix + 1;
-            const int xpp = xp + 1 == NX ? 0 : xp + 1;
-            const int ym = iy == 0 ? NY - 1 : iy - 1, yp = iy + 1 == NY ? 0 : iy + 1;
-            const int ypp = yp + 1 == NY ? 0 : yp + 1;
-            const size_t pl = (size_t)iz * NXY;
-            const size_t r0 = pl + (size_t)iy * NX, rm = pl + (size_t)ym * NX, rp = pl + (size_t)yp * NX,
-                         rpp = pl + (size_t)ypp * NX;
-            const bool lo = iz > 0, hi = iz + 1 < NZ;
-            const size_t dm = lo ? NXY : 0, dp = hi ? NXY : 0;
-            // cell-centred values: u_c = (u_x + u_{x+1})/2, v_c = (v_y + v_{y+1})/2,
-            // w_c = (w_z + w_{z+1})/2 (w_NZ = 0); central differences, the wall value 0
-            // replacing a missing z-neighbour
-            float G[3][3];
-            G[0][0] = (float)((u[r0 + xpp] + u[r0 + xp]) - (u[r0 + ix] + u[r0 + xm])) * gx;
-            G[0][1] = (float)((u[rp + ix] + u[rp + xp]) - (u[rm + ix] + u[rm + xp])) * gy;
-            G[1][0] = (float)((v[r0 + xp] + v[rp + xp]) - (v[r0 + xm] + v[rp + xm])) * gx;
-            G[1][1] = (float)((v[rpp + ix] + v[rp + ix]) - (v[r0 + ix] + v[rm + ix])) * gy;
-            const T w0 = w[r0 + ix], w1 = hi ? w[r0 + ix + NXY] : T(0);
-            G[2][0] = (float)((w[r0 + xp] + (hi ? w[r0 + xp + NXY] : T(0))) -
-                              (w[r0 + xm] + (hi ? w[r0 + xm + NXY] : T(0)))) * gx;
-            G[2][1] = (float)((w[rp + ix] + (hi ? w[rp + ix + NXY] : T(0))) -
-                              (w[rm + ix] + (hi ? w[rm + ix + NXY] : T(0)))) * gy;
-            // z: (q(z+1) - q(z-1)) / (zc(z+1) - zc(z-1)) with zc the wall plane at a wall
-            const double zm = lo ? 0.5 * (ZZ[iz - 1] + ZZ[iz]) : ZZ[0];
-            const double zp = hi ? 0.5 * (ZZ[iz + 1] + ZZ[iz + 2]) : ZZ[NZ];
-            const float gz = (float)(0.5 / (zp - zm));
-            const T uzp = hi ? u[r0 + ix + dp] + u[r0 + xp + dp] : T(0);
-            const T uzm = lo ? u[r0 + ix - dm] + u[r0 + xp - dm] : T(0);
-            const T vzp = hi ? v[r0 + ix + dp] + v[rp + ix + dp] : T(0);
-            const T vzm = lo ? v[r0 + ix - dm] + v[rp + ix - dm] : T(0);
-            const T wzp = hi ? w1 + (iz + 2 < NZ ? w[r0 + ix + 2 * NXY] : T(0)) : T(0);
-            const T wzm = lo ? w[r0 + ix - NXY] + w0 : T(0);
-            G[0][2] = (float)(uzp - uzm) * gz;
-            G[1][2] = (float)(vzp - vzm) * gz;
-            G[2][2] = (float)(wzp - wzm) * gz;
-            const double zc = 0.5 * (ZZ[iz] + ZZ[iz + 1]);
-            const double d = fmin(zc - ZZ[0], ZZ[NZ] - zc);
-            les_features_f(G, sc, (float)(d * utau / nu), Xs[wid][lane]);
+            les_features_bf16(G, sc, (float)a.m.LYP[iz], &Xb[wid][lane][0]);
+        } else {
+            *reinterpret_cast<uint4*>(&Xb[wid][lane][0]) = make_uint4(0u, 0u, 0u, 0u);
         }
         __syncwarp();
-#pragma unroll 1
-        for (int h = 0; h < 2; h++) {
-            const int nr = min(16, nrow - 16 * h);
-            if (nr <= 0) break;
-            unsigned ax[4];
-            feature_fragment(&Xs[wid][16 * h][0], MLP_IN, nr, ax);
-            Acc64 z1, z2;
-            unsigned h1a[4][4];
-            float z3[2];
-            mlp_forward_tile(S, ax, z1, z2, h1a, z3);
-            if (t == 0) {
-                const long long cb = c0 + 16 * h;
-                const long long top = COLL ? (long long)(NZ - 1) * (long long)NXY : N;  // first cell without element
-                if (gq < nr && cb + gq < top) a.nu_t[cb + gq] = (T)(nu * softplus(z3[0]));
-                if (gq + 8 < nr && cb + gq + 8 < top) a.nu_t[cb + gq + 8] = (T)(nu * softplus(z3[1]));
-            }
-        }
+        const float z3 = mlp_infer32(S, Xb[wid]);
+        const unsigned cl = c0 + 16u * (t >> 1) + 8u * (t & 1) + gq;
+        if (cl < top) a.nu_t[cl] = (T)(g.visc * softplus(z3));
         __syncwarp();
     }
 }
@@ -301,7 +272,7 @@ void launch_les_features(const float* F, const Geom& g, int fw, int fz, const do
 template <typename T>
 void launch_turb_mlp(const TurbArgs<T>& a, const float* P, cudaStream_t s) {
     const long long ngrp = (a.g.N + 31) / 32;
-    const int nb = (int)std::max<long long>(1, std::min<long long>((ngrp + 3) / 4, 148 * 6));
+    const int nb = (int)std::max<long long>(1, std::min<long long>((ngrp + 3) / 4, 148 * 4));  // one wave
     if (a.g.scheme == TC_SCHEME_COLLOC) k_turb_mlp<T, true><<<nb, 128, 0, s>>>(a, P);
     else k_turb_mlp<T, false><<<nb, 128, 0, s>>>(a, P);
 }

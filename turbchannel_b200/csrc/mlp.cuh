@@ -102,44 +102,6 @@ __device__ __forceinline__ float dsilu(float z) {
 }
 __device__ __forceinline__ float softplus(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
-// The closure's inputs in float (the run's inference path; the training samples use
-// les_features in double): same invariants, then rounded to BF16 by the network.
-__device__ __forceinline__ void les_features_f(const float G[3][3], float sc, float yplus, float* f) {
-    float S[3][3], O[3][3];
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            S[i][j] = 0.5f * (G[i][j] + G[j][i]) * sc;
-            O[i][j] = 0.5f * (G[i][j] - G[j][i]) * sc;
-        }
-    float S2[3][3], O2[3][3];
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            S2[i][j] = S[i][0] * S[0][j] + S[i][1] * S[1][j] + S[i][2] * S[2][j];
-            O2[i][j] = O[i][0] * O[0][j] + O[i][1] * O[1][j] + O[i][2] * O[2][j];
-        }
-    float l1 = 0, l2 = 0, l3 = 0, l4 = 0, l5 = 0;
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            l1 += S[i][j] * S[j][i];
-            l2 += O[i][j] * O[j][i];
-            l3 += S2[i][j] * S[j][i];
-            l4 += O2[i][j] * S[j][i];
-            l5 += O2[i][j] * S2[j][i];
-        }
-    f[0] = asinhf(l1);
-    f[1] = asinhf(l2);
-    f[2] = asinhf(l3);
-    f[3] = asinhf(l4);
-    f[4] = asinhf(l5);
-    f[5] = 0.25f * log1pf(yplus);
-}
-
 // Accumulator tile 16 x 64: 8 n-tiles of m16n8, element (row g or g+8, col 8 nt + 2t (+1)).
 struct Acc64 {
     float c[8][4];
@@ -154,6 +116,123 @@ __device__ __forceinline__ void c_to_a(const Acc64& C, unsigned A[4][4]) {
         A[kk][2] = pack_bf16(C.c[2 * kk + 1][0], C.c[2 * kk + 1][1]);
         A[kk][3] = pack_bf16(C.c[2 * kk + 1][2], C.c[2 * kk + 1][3]);
     }
+}
+
+// ---- inference of 32 samples ----
+__device__ __forceinline__ float ex2_fast(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rcp_fast(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+// silu of two values with one reciprocal: 1/(1+a) = (1+b) / ((1+a)(1+b)), a = e^-z0, b = e^-z1.
+// Three special-function operations for two values instead of four, at an error of two more
+// roundings (float ulps, below the BF16 rounding that follows); a, b are held below 2^63 so
+// that the product stays finite (silu below z = -44 is then -z 2^-63 instead of less).
+__device__ __forceinline__ float2 silu2(float z0, float z1) {
+    const float L2E = 1.44269504088896340736f;
+    const float2 t = __fmul2_rn(make_float2(z0, z1), make_float2(-L2E, -L2E));
+    const float2 d = __fadd2_rn(make_float2(ex2_fast(fminf(t.x, 63.f)), ex2_fast(fminf(t.y, 63.f))), make_float2(1.f, 1.f));
+    const float r = rcp_fast(d.x * d.y);
+    return __fmul2_rn(make_float2(z0, z1), __fmul2_rn(make_float2(r, r), make_float2(d.y, d.x)));
+}
+// B fragments of two k-steps (kk, kk+1) of n-tile nt from a [n][k] bf16 array in one ldmatrix.
+template <int LD>
+__device__ __forceinline__ void ldb2(const __nv_bfloat16 (*M)[LD], int kk, int nt, unsigned b[4]) {
+    const int lane = threadIdx.x & 31;
+    const unsigned a = smem_u32(&M[nt * 8 + (lane & 7)][kk * 16 + 8 * (lane >> 3)]);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3])
+                 : "r"(a));
+}
+
+// Forward pass of 32 samples (two 16-row tiles sharing every weight fragment) whose features
+// lie in xb as bf16 [sample][8] (6 features, 2 zeros).  Returns z3 of the sample this lane
+// stands for: 16 (t >> 1) + 8 (t & 1) + g with g = lane / 4, t = lane % 4.
+__device__ __forceinline__ float mlp_infer32(const MlpSmem& S, const __nv_bfloat16 (*xb)[8]) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    unsigned ax[2][2];
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) ax[m][h] = *reinterpret_cast<const unsigned*>(&xb[16 * m + 8 * h + g][2 * t]);
+    unsigned h1[2][4][4];
+#pragma unroll
+    for (int nt = 0; nt < 8; nt++) {
+        const float2 b = *reinterpret_cast<const float2*>(&S.b1[8 * nt + 2 * t]);
+        const unsigned w0 = *reinterpret_cast<const unsigned*>(&S.W1T[nt * 8 + g][2 * t]);
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+            float z[4] = {b.x, b.y, b.x, b.y};
+            const unsigned a[4] = {ax[m][0], ax[m][1], 0u, 0u};  // features k >= 8 are zero, and so is their weight row
+            mma_bf16(z, a, w0, 0u);
+            const float2 lo = silu2(z[0], z[1]), hi = silu2(z[2], z[3]);
+            h1[m][nt >> 1][2 * (nt & 1)] = pack_bf16(lo.x, lo.y);
+            h1[m][nt >> 1][2 * (nt & 1) + 1] = pack_bf16(hi.x, hi.y);
+        }
+    }
+    float p[2][2] = {};
+#pragma unroll
+    for (int nt = 0; nt < 8; nt++) {
+        unsigned w[2][4];
+        ldb2<MLP_LD2>(S.W2T, 0, nt, w[0]);
+        ldb2<MLP_LD2>(S.W2T, 2, nt, w[1]);
+        const float2 b = *reinterpret_cast<const float2*>(&S.b2[8 * nt + 2 * t]);
+        const float2 w3 = *reinterpret_cast<const float2*>(&S.w3[8 * nt + 2 * t]);
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+            float z[4] = {b.x, b.y, b.x, b.y};
+#pragma unroll
+            for (int kk = 0; kk < 4; kk++) mma_bf16(z, h1[m][kk], w[kk >> 1][2 * (kk & 1)], w[kk >> 1][2 * (kk & 1) + 1]);
+            const float2 lo = silu2(z[0], z[1]), hi = silu2(z[2], z[3]);
+            const __nv_bfloat162 l = __floats2bfloat162_rn(lo.x, lo.y), h = __floats2bfloat162_rn(hi.x, hi.y);
+            p[m][0] += w3.x * __low2float(l);
+            p[m][0] += w3.y * __high2float(l);
+            p[m][1] += w3.x * __low2float(h);
+            p[m][1] += w3.y * __high2float(h);
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            p[m][h] += __shfl_xor_sync(0xffffffffu, p[m][h], 1);
+            p[m][h] += __shfl_xor_sync(0xffffffffu, p[m][h], 2);
+        }
+    const float q0 = (t & 1) ? p[0][1] : p[0][0], q1 = (t & 1) ? p[1][1] : p[1][0];
+    return ((t & 2) ? q1 : q0) + S.b3;
+}
+
+// The closure's inputs in float (the run's inference path; the training samples use
+// les_features in double), as the network's BF16 inputs: the five invariants of S and O from
+// the unique entries of the symmetric S and the antisymmetric O = {O01, O02, O12} (sc: the
+// wall-unit scale), and the plane's y+ input.
+__device__ __forceinline__ void les_features_bf16(const float G[3][3], float sc, float yp, __nv_bfloat16* out) {
+    const float h = 0.5f * sc;
+    const float s00 = G[0][0] * sc, s11 = G[1][1] * sc, s22 = G[2][2] * sc;
+    const float s01 = (G[0][1] + G[1][0]) * h, s02 = (G[0][2] + G[2][0]) * h, s12 = (G[1][2] + G[2][1]) * h;
+    const float a = (G[0][1] - G[1][0]) * h, b = (G[0][2] - G[2][0]) * h, c = (G[1][2] - G[2][1]) * h;
+    // S^2 and O^2 (both symmetric)
+    const float t00 = s00 * s00 + s01 * s01 + s02 * s02, t11 = s01 * s01 + s11 * s11 + s12 * s12,
+                t22 = s02 * s02 + s12 * s12 + s22 * s22;
+    const float t01 = s00 * s01 + s01 * s11 + s02 * s12, t02 = s00 * s02 + s01 * s12 + s02 * s22,
+                t12 = s01 * s02 + s11 * s12 + s12 * s22;
+    const float o00 = -(a * a + b * b), o11 = -(a * a + c * c), o22 = -(b * b + c * c);
+    const float o01 = -b * c, o02 = a * c, o12 = -a * b;
+    const float l1 = t00 + t11 + t22, l2 = o00 + o11 + o22;
+    const float l3 = t00 * s00 + t11 * s11 + t22 * s22 + 2.f * (t01 * s01 + t02 * s02 + t12 * s12);
+    const float l4 = o00 * s00 + o11 * s11 + o22 * s22 + 2.f * (o01 * s01 + o02 * s02 + o12 * s12);
+    const float l5 = o00 * t00 + o11 * t11 + o22 * t22 + 2.f * (o01 * t01 + o02 * t02 + o12 * t12);
+    uint4 v;
+    v.x = pack_bf16(asinhf(l1), asinhf(l2));
+    v.y = pack_bf16(asinhf(l3), asinhf(l4));
+    v.z = pack_bf16(asinhf(l5), yp);
+    v.w = 0u;
+    *reinterpret_cast<uint4*>(out) = v;
 }
 
 // Forward pass of one 16-sample tile.  ax: A fragment of the features (16 x 16).

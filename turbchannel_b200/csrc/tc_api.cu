@@ -291,7 +291,7 @@ static MeshDev<T> mesh_dev(const tc_handle* h) {
     MeshDev<T> m;
     m.ZZ = t + 0 * L; m.DZ = t + 1 * L; m.DZW = t + 2 * L; m.GC1 = t + 3 * L; m.GC2 = t + 4 * L;
     m.GCZ = t + 5 * L; m.KERG = t + 6 * L; m.cellh = t + 7 * L; m.MAT_A = t + 8 * L; m.PC = t + 11 * L;
-    m.SM = t + (11 + TC_PC) * L;
+    m.SM = t + (11 + TC_PC) * L; m.LGZ = t + (12 + TC_PC) * L; m.LYP = t + (13 + TC_PC) * L;
     m.FK = h->fp64 ? nullptr : (const float*)h->fk;
     m.FK64 = h->fp64 ? (const double*)h->fk : nullptr;
     m.dZZ = d + 0 * L; m.dDZ = d + 1 * L; m.dDZW = d + 2 * L; m.dKERG = d + 6 * L; m.dcellh = d + 7 * L;
@@ -392,6 +392,27 @@ static void fill_smagorinsky(const Geom& g, const HostMesh& hm, double* sm) {
         const double fvd = 1 - std::exp(-(0.04 * 0.04 * 0.04) * yp * yp * yp);
         const double Dl = std::min(0.1 * std::pow(g.hx * g.hy * hm.DZ[z], 0.33333333333333333333), 0.41 * d);
         sm[z] = fvd * Dl * Dl;
+    }
+}
+
+// The learned closure's per-plane constants: gz, the factor of the difference of (sums of
+// two or four) values above and below (staggered: central over the neighbouring centres, the
+// wall closing it; collocated: over the element), and 0.25 log(1 + y+).
+static void fill_closure(const Geom& g, const HostMesh& hm, double* gz, double* yp) {
+    const bool coll = g.scheme == TC_SCHEME_COLLOC;
+    const std::vector<double>& ZZ = hm.ZZ;
+    const int nl = coll ? g.NZ - 1 : g.NZ;
+    const double utau = g.inv_ls * g.visc;
+    for (int z = 0; z < nl; z++) {
+        if (coll) gz[z] = (double)(float)(0.25 / (ZZ[z + 1] - ZZ[z]));
+        else {
+            const double zm = z > 0 ? 0.5 * (ZZ[z - 1] + ZZ[z]) : ZZ[0];
+            const double zp = z + 1 < nl ? 0.5 * (ZZ[z + 1] + ZZ[z + 2]) : ZZ[nl];
+            gz[z] = (double)(float)(0.5 / (zp - zm));
+        }
+        const double zc = 0.5 * (ZZ[z] + ZZ[z + 1]);
+        const double d = std::fmin(zc - ZZ[0], ZZ[nl] - zc);
+        yp[z] = (double)(0.25f * log1pf((float)(d * utau / g.visc)));
     }
 }
 
@@ -520,9 +541,9 @@ extern "C" int tc_create(const tc_params* prm, const double* zz, tc_handle** out
     TC_ALLOC(h->zfac, zfactor_bytes(g, (int)E));
     if (!h->fp64) TC_ALLOC(h->zfac_low, zfactor_low_bytes(g));
     // mesh arrays, 9 slots of NZ+2 (the last one holds MAT_A, up to 3 NZ entries), then
-    // the per-plane reciprocals (TC_PC per plane) and the Smagorinsky factor (one per plane)
+    // the per-plane reciprocals (TC_PC per plane) the Smagorinsky factor and the closure's two constants (one per plane each)
     const int L = g.NZ + 2;
-    const size_t mlen = (size_t)8 * L + 3 * (size_t)L + (size_t)TC_PC * L + (size_t)L;
+    const size_t mlen = (size_t)8 * L + 3 * (size_t)L + (size_t)TC_PC * L + (size_t)3 * L;
     TC_ALLOC(h->mesh_t, mlen * E);
     TC_ALLOC(h->mesh_d, mlen * sizeof(double));
     {
@@ -536,6 +557,7 @@ extern "C" int tc_create(const tc_params* prm, const double* zz, tc_handle** out
         const size_t pc0 = (size_t)11 * L;
         fill_plane_consts<double>(g, hm, md.data(), md.data() + pc0);
         fill_smagorinsky(g, hm, md.data() + pc0 + (size_t)TC_PC * L);
+        fill_closure(g, hm, md.data() + pc0 + (size_t)(TC_PC + 1) * L, md.data() + pc0 + (size_t)(TC_PC + 2) * L);
         if (cudaMemcpy(h->mesh_d, md.data(), mlen * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) {
             free_all(h); delete h;
             return fail(TC_E_CUDA, "tc_create: mesh upload failed");

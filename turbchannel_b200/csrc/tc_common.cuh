@@ -39,6 +39,9 @@ constexpr int TC_FK = 48, TC_FK64 = 24;
 template <typename T>
 struct MeshDev {
     const T *ZZ, *DZ, *DZW, *GC1, *GC2, *GCZ, *KERG, *MAT_A, *cellh, *PC;
+    // learned closure, per plane of cells or layer of elements: the z-difference factor of the
+    // gradient and the y+ input 0.25 log(1 + y+) (float values)
+    const T *LGZ = nullptr, *LYP = nullptr;
     const T* SM = nullptr;  // Smagorinsky-van Driest: nu_t / |S| of each plane (staggered) or element layer (collocated)
     const float* FK = nullptr;
     const double* FK64 = nullptr;

@@ -3,8 +3,8 @@
 // N = N1 * N2 (Cooley-Tukey, n = N2*n1 + n2, k = k1 + N1*k2):
 //   pass A  one item per (line, n2): the thread holds x[N2*n1 + n2], n1 < N1, does a
 //           length-N1 DFT in registers, multiplies by W_N^(n2*k1) and writes
-//           Y[k1][n2] to shared memory (row stride N2+1, which keeps the column reads
-//           of pass B free of bank conflicts);
+//           Y[k1][n2] to shared memory (row stride ST = N2+1, N2+2 for odd N2: an odd
+//           stride keeps the column reads of pass B free of bank conflicts);
 //   pass B  one item per (line, k1): the thread reads Y[k1][0..N2), does a length-N2
 //           DFT in registers and holds X[k1 + N1*k2], k2 < N2.
 // The register DFTs are mixed radix-4/2/3 with every inner twiddle a compile-time
@@ -130,20 +130,39 @@ struct FftSplit {
     struct FftSplit<n> {                          \
         static constexpr bool ok = true;          \
         static constexpr int N1 = a, N2 = b;      \
-        static constexpr int YL = a * (b + 1);    \
+        static constexpr int ST = b + 1 + b % 2;  \
+        static constexpr int YL = a * ST;         \
     };
+TC_FFT_SPLIT(8, 2, 4)
+TC_FFT_SPLIT(12, 3, 4)
 TC_FFT_SPLIT(16, 4, 4)
+TC_FFT_SPLIT(18, 3, 6)
 TC_FFT_SPLIT(24, 4, 6)
 TC_FFT_SPLIT(32, 4, 8)
+TC_FFT_SPLIT(36, 6, 6)
 TC_FFT_SPLIT(48, 6, 8)
+TC_FFT_SPLIT(54, 6, 9)
 TC_FFT_SPLIT(64, 8, 8)
+TC_FFT_SPLIT(72, 8, 9)
 TC_FFT_SPLIT(96, 8, 12)
+TC_FFT_SPLIT(108, 9, 12)
 TC_FFT_SPLIT(128, 8, 16)
+TC_FFT_SPLIT(144, 12, 12)
+TC_FFT_SPLIT(162, 9, 18)
 TC_FFT_SPLIT(192, 12, 16)
+TC_FFT_SPLIT(216, 12, 18)
 TC_FFT_SPLIT(256, 16, 16)
+TC_FFT_SPLIT(288, 16, 18)
+TC_FFT_SPLIT(324, 18, 18)
 TC_FFT_SPLIT(384, 16, 24)
+TC_FFT_SPLIT(432, 18, 24)
+TC_FFT_SPLIT(486, 18, 27)
 TC_FFT_SPLIT(512, 16, 32)
+TC_FFT_SPLIT(576, 24, 24)
+TC_FFT_SPLIT(648, 24, 27)
 TC_FFT_SPLIT(768, 24, 32)
+TC_FFT_SPLIT(864, 27, 32)
+TC_FFT_SPLIT(972, 27, 36)
 TC_FFT_SPLIT(1024, 32, 32)
 #undef TC_FFT_SPLIT
 
@@ -162,14 +181,14 @@ __device__ __forceinline__ cplx<T> ldg_c(const cplx<T>* p) {
 template <typename T, int N, int SIGN>
 __device__ __forceinline__ void fft_pass_a(cplx<T> (&v)[FftSplit<N>::N1], int n2, const cplx<T>* __restrict__ tw,
                                            cplx<T>* Yl) {
-    constexpr int N1 = FftSplit<N>::N1, N2 = FftSplit<N>::N2;
+    constexpr int N1 = FftSplit<N>::N1;
     rdft<T, N1, SIGN>(v);
     Yl[n2] = v[0];
 #pragma unroll
     for (int k1 = 1; k1 < N1; k1++) {
         cplx<T> w = ldg_c(tw + n2 * k1);
         if (SIGN > 0) w.y = -w.y;
-        Yl[k1 * (N2 + 1) + n2] = cmul(v[k1], w);
+        Yl[k1 * FftSplit<N>::ST + n2] = cmul(v[k1], w);
     }
 }
 
@@ -177,7 +196,7 @@ __device__ __forceinline__ void fft_pass_a(cplx<T> (&v)[FftSplit<N>::N1], int n2
 template <typename T, int N, int SIGN>
 __device__ __forceinline__ void fft_pass_b(cplx<T> (&v)[FftSplit<N>::N2], int k1, const cplx<T>* Yl) {
     constexpr int N2 = FftSplit<N>::N2;
-    const cplx<T>* row = Yl + k1 * (N2 + 1);
+    const cplx<T>* row = Yl + k1 * FftSplit<N>::ST;
 #pragma unroll
     for (int n2 = 0; n2 < N2; n2++) v[n2] = row[n2];
     rdft<T, N2, SIGN>(v);

@@ -1,78 +1,12 @@
-// k_fft.cu -- the pressure solve's FFT kernels for the lengths that have a compiled
-// two-pass register transform (fft_reg.cuh: 16 ... 1024 = 2^a 3^b); other lengths
-// keep the Stockham kernels of k_poisson.cu.  Same data layouts and results:
+// k_fft.cu -- the divergence kernel and the dispatch of the pressure solve's register FFTs
+// (k_fft.cuh) by transform length; lengths without one keep the Stockham kernels of
+// k_poisson.cu.  Same data layouts and results.
 //   k_div_quad_z   : divergence of the vector RHS (streaming, 16-byte row loads)
-//                    into a scratch real field;
-//   k_xfft_reg     : forward x-FFT of `rows` y-rows of a real field (the divergence
-//                    or the scalar RHS), two rows packed as one complex line,
-//                    unpacked to spec[z][kx][y] (kx = 0..NX/2);
-//   k_yfft_reg     : complex FFT of contiguous y-lines of spec, in place, straight
-//                    from and back to global memory;
-//   k_ixfft_reg    : Hermitian-extended half spectrum of two rows packed as one
-//                    complex line, inverse x-FFT, scaled real rows into p.
-#include <algorithm>
-
-#include "fft_reg.cuh"
-#include "kernels.cuh"
+//                    into a scratch real field.
+#include "k_fft.cuh"
 #include "stencil_div.cuh"
 
 namespace tc {
-
-// ---------------------------------------------------------------------------
-// y-FFT
-// ---------------------------------------------------------------------------
-constexpr int YFFT_LINE_BUDGET = 128;  // lines x N1 per CTA
-// Lines per CTA: few (8 at N = 384: 26 KB of shared memory in float, 51 KB in double),
-// so that many CTAs share an SM and hide each other's global-memory latency (measured
-// at 384 x 384 x 256: 32 float lines per CTA 0.082 ms, 16 lines 0.074, 8 lines 0.058).
-template <typename T, int N>
-constexpr int yfft_reg_lines() {
-    const int l = YFFT_LINE_BUDGET / FftSplit<N>::N1;
-    return l < 1 ? 1 : l;
-}
-
-template <typename T, int N, int SIGN>
-__global__ void __launch_bounds__(256) k_yfft_reg(cplx<T>* spec, long long nlines, const cplx<T>* __restrict__ tw) {
-    constexpr int N1 = FftSplit<N>::N1, N2 = FftSplit<N>::N2, YL = FftSplit<N>::YL;
-    constexpr int LINES = yfft_reg_lines<T, N>();
-    extern __shared__ __align__(16) unsigned char smraw[];
-    cplx<T>* Y = reinterpret_cast<cplx<T>*>(smraw);
-    // the forward transform takes the lines in descending z, the reverse of the x-FFT that
-    // wrote them (its last planes are still in L2), and leaves the low planes, which the
-    // z-solve's forward sweep reads first, written last (384x256x384 float: y-FFT 0.052
-    // against 0.059 ms, z-solve 0.144 against 0.152; double 0.097 / 0.283 against 0.101 / 0.292)
-    const long long blk = SIGN < 0 ? (long long)gridDim.x - 1 - blockIdx.x : (long long)blockIdx.x;
-    const long long L0 = blk * LINES;
-    const int nl = (int)min((long long)LINES, nlines - L0);
-    cplx<T>* base = spec + L0 * N;
-    for (int it = threadIdx.x; it < nl * N2; it += blockDim.x) {
-        const int l = it / N2, n2 = it - l * N2;
-        const cplx<T>* src = base + (size_t)l * N + n2;
-        cplx<T> v[N1];
-#pragma unroll
-        for (int n1 = 0; n1 < N1; n1++) v[n1] = src[n1 * N2];
-        fft_pass_a<T, N, SIGN>(v, n2, tw, Y + l * YL);
-    }
-    __syncthreads();
-    for (int it = threadIdx.x; it < nl * N1; it += blockDim.x) {
-        const int l = it / N1, k1 = it - l * N1;
-        cplx<T> v[N2];
-        fft_pass_b<T, N, SIGN>(v, k1, Y + l * YL);
-        cplx<T>* dst = base + (size_t)l * N + k1;
-#pragma unroll
-        for (int k2 = 0; k2 < N2; k2++) dst[k2 * N1] = v[k2];
-    }
-}
-
-template <typename T, int N>
-static void yfft_reg_launch(const YFftArgs<T>& a, cudaStream_t s) {
-    constexpr int LINES = yfft_reg_lines<T, N>();
-    const long long total = (long long)a.g.NZ * a.g.NXH;
-    const size_t smem = (size_t)LINES * FftSplit<N>::YL * sizeof(cplx<T>);
-    auto k = a.sign < 0 ? k_yfft_reg<T, N, -1> : k_yfft_reg<T, N, +1>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k<<<(unsigned)((total + LINES - 1) / LINES), 256, smem, s>>>(a.spec, total, a.twy);
-}
 
 // ---------------------------------------------------------------------------
 // divergence of the vector RHS (streaming, 4 cells of a row per thread) and the
@@ -185,207 +119,6 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 3 : 4) k_div_quad_z(DivF
     }
 }
 
-// Whether the forward x-FFT of `rows` rows (256 threads) keeps its transformed lines in
-// the first pass's buffer: one second-pass line segment per thread at most.
-template <int N>
-__host__ __device__ constexpr bool xfft_alias(int rows) {
-    return (rows / 2) * FftSplit<N>::N1 <= 256;
-}
-
-// Three CTAs per SM in float (79 registers at N = 384, no spill), two in double.
-template <typename T, int N>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_xfft_reg(DivFftArgs<T> a, const T* __restrict__ src, int rows, int lrows) {
-    constexpr int N1 = FftSplit<N>::N1, N2 = FftSplit<N>::N2, YL = FftSplit<N>::YL, ZS = N + 1;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    const Geom& g = a.g;
-    const int NY = g.NY, NXH = N / 2 + 1, nl = rows >> 1;
-    cplx<T>* Y = reinterpret_cast<cplx<T>*>(smraw);
-    // transformed lines, stride N+1: over Y itself when every thread holds at most one
-    // line segment of the second pass (read all, barrier, write), else after Y
-    const bool alias = xfft_alias<N>(rows);
-    cplx<T>* Zs = alias ? Y : Y + nl * YL;
-    const int z = blockIdx.y, y0 = blockIdx.x * rows;
-    const T* plane = src + ((size_t)z * NY + y0) * N;
-    for (int it = threadIdx.x; it < nl * N2; it += blockDim.x) {
-        const int l = it / N2, n2 = it - l * N2;
-        const T* d0 = plane + (size_t)(2 * l) * N + n2;
-        cplx<T> v[N1];
-#pragma unroll
-        for (int n1 = 0; n1 < N1; n1++) v[n1] = {__ldg(d0 + n1 * N2), __ldg(d0 + N + n1 * N2)};
-        fft_pass_a<T, N, -1>(v, n2, a.twx, Y + l * YL);
-    }
-    __syncthreads();
-    if (alias) {
-        const bool mine = (int)threadIdx.x < nl * N1;
-        const int l = threadIdx.x / N1, k1 = threadIdx.x - l * N1;
-        cplx<T> v[N2];
-        if (mine) fft_pass_b<T, N, -1>(v, k1, Y + l * YL);
-        __syncthreads();
-        if (mine) {
-            cplx<T>* zl = Zs + l * ZS + k1;
-#pragma unroll
-            for (int k2 = 0; k2 < N2; k2++) zl[k2 * N1] = v[k2];
-        }
-    } else {
-        for (int it = threadIdx.x; it < nl * N1; it += blockDim.x) {
-            const int l = it / N1, k1 = it - l * N1;
-            cplx<T> v[N2];
-            fft_pass_b<T, N, -1>(v, k1, Y + l * YL);
-            cplx<T>* zl = Zs + l * ZS + k1;
-#pragma unroll
-            for (int k2 = 0; k2 < N2; k2++) zl[k2 * N1] = v[k2];
-        }
-    }
-    __syncthreads();
-    // unpack the two real rows of each line: X_a = (Z_k + conj Z_{N-k}) / 2, X_b = (Z_k - conj Z_{N-k}) / 2i
-    for (int e = threadIdx.x; e < NXH * rows; e += blockDim.x) {
-        const int kx = e >> lrows, r = e & (rows - 1), l = r >> 1;
-        const cplx<T> Zk = Zs[l * ZS + kx], Zm = Zs[l * ZS + (kx == 0 ? 0 : N - kx)];
-        cplx<T> val;
-        if ((r & 1) == 0) val = {T(0.5) * (Zk.x + Zm.x), T(0.5) * (Zk.y - Zm.y)};
-        else val = {T(0.5) * (Zk.y + Zm.y), -T(0.5) * (Zk.x - Zm.x)};
-        a.spec[((size_t)z * NXH + kx) * NY + y0 + r] = val;
-    }
-}
-
-template <typename T, int N>
-static size_t div_xfft_reg_smem(int rows) {
-    return (size_t)(rows / 2) * (FftSplit<N>::YL + (xfft_alias<N>(rows) ? 0 : N + 1)) * sizeof(cplx<T>);
-}
-
-template <typename T, int N>
-static void xfft_reg_launch(const DivFftArgs<T>& a, const T* src, int rows, cudaStream_t s) {
-    const size_t smem = div_xfft_reg_smem<T, N>(rows);
-    int lr = 0;
-    while ((1 << lr) < rows) lr++;
-    auto k = k_xfft_reg<T, N>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k<<<dim3(a.g.NY / rows, a.g.NZ), 256, smem, s>>>(a, src, rows, lr);
-}
-
-// ---------------------------------------------------------------------------
-// inverse x-FFT, persistent and double-buffered (float)
-// ---------------------------------------------------------------------------
-constexpr int XP_NT = 256;
-// As k_ixfft_reg (the Hermitian-extended
-// half spectrum of two rows per complex line, inverse transform, scaled rows into p), with
-// each CTA walking tiles of RB (16) y-values of one plane and copying the next tile's half
-// spectrum (NX/2+1 rows of RB contiguous values) into its second buffer while it
-// transforms the current one.
-template <typename T, int N>
-struct IPipe {
-    static constexpr int RB = sizeof(T) == 4 ? 16 : 8, NL = RB / 2, TS = RB + 2, NXH = N / 2 + 1;
-    static constexpr int PC = 16 / sizeof(cplx<T>), CPK = RB / PC;  // 16-byte chunks per kx row
-    static constexpr size_t buf = ((size_t)NXH * TS * sizeof(cplx<T>) + 15) / 16 * 16;
-    static constexpr size_t smem = 2 * buf + (size_t)NL * FftSplit<N>::YL * sizeof(cplx<T>);
-};
-
-template <typename T, int N>
-__global__ void __launch_bounds__(XP_NT) k_ixfft_pipe(IxFftArgs<T> a) {
-    using P = IPipe<T, N>;
-    constexpr int RB = P::RB, NL = P::NL, TS = P::TS, NXH = P::NXH, PC = P::PC, CPK = P::CPK;
-    constexpr int N1 = FftSplit<N>::N1, N2 = FftSplit<N>::N2, YL = FftSplit<N>::YL, NH = N / 2;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    cplx<T>* Y = reinterpret_cast<cplx<T>*>(smraw + 2 * P::buf);
-    const Geom& g = a.g;
-    const int NY = g.NY, YB = NY / RB;
-    const long long ntile = (long long)YB * g.NZ;
-    // tiles in ascending z: the correction that reads p next walks the planes downwards,
-    // so that the next step's flux kernel, which starts at z = 0, finds the low planes of
-    // the new velocity in L2 (at 384x256x384 the flux kernel gains more, 7 us, than this
-    // kernel loses against descending tiles, 1.5 us)
-    auto fetch = [&](long long t, int b) {
-        const int z = (int)(t / YB), y0 = (int)(t - (long long)z * YB) * RB;
-        cplx<T>* tile = reinterpret_cast<cplx<T>*>(smraw + b * P::buf);
-        for (int e = threadIdx.x; e < NXH * CPK; e += XP_NT) {
-            const int kx = e / CPK, c = e - kx * CPK;
-            cp_async<16>(tile + kx * TS + c * PC, a.spec + ((size_t)z * NXH + kx) * NY + y0 + c * PC);
-        }
-    };
-    long long t = blockIdx.x;
-    if (t < ntile) fetch(t, 0);
-    cp_async_commit();
-    const T sc = a.scale;
-    for (int b = 0; t < ntile; t += gridDim.x, b ^= 1) {
-        if (t + gridDim.x < ntile) fetch(t + gridDim.x, b ^ 1);
-        cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();  // tile t is in buffer b
-        const int z = (int)(t / YB), y0 = (int)(t - (long long)z * YB) * RB;
-        const cplx<T>* tile = reinterpret_cast<const cplx<T>*>(smraw + b * P::buf);
-        for (int it = threadIdx.x; it < NL * N2; it += XP_NT) {
-            const int l = it / N2, n2 = it - l * N2;
-            cplx<T> v[N1];
-#pragma unroll
-            for (int n1 = 0; n1 < N1; n1++) {  // the Hermitian-extended line of rows 2l, 2l+1
-                const int k = N2 * n1 + n2;
-                const bool up = k > NH;
-                const cplx<T>* tp = tile + (up ? N - k : k) * TS + 2 * l;
-                cplx<T> av = tp[0], bv = tp[1];
-                if (up) {
-                    av.y = -av.y;
-                    bv.y = -bv.y;
-                }
-                if (k == 0 || k == NH) {
-                    av.y = 0;
-                    bv.y = 0;
-                }
-                v[n1] = {av.x - bv.y, av.y + bv.x};
-            }
-            fft_pass_a<T, N, +1>(v, n2, a.twx, Y + l * YL);
-        }
-        __syncthreads();
-        for (int it = threadIdx.x; it < NL * N1; it += XP_NT) {
-            const int l = it / N1, k1 = it - l * N1;
-            cplx<T> v[N2];
-            fft_pass_b<T, N, +1>(v, k1, Y + l * YL);
-            T* pa = a.p + ((size_t)z * NY + y0 + 2 * l) * N + k1;
-            T* pb = pa + N;
-#pragma unroll
-            for (int k2 = 0; k2 < N2; k2++) {
-                pa[k2 * N1] = v[k2].x * sc;
-                pb[k2 * N1] = v[k2].y * sc;
-            }
-        }
-        __syncthreads();  // buffer b and Y are refilled by the next iterations
-    }
-}
-
-template <typename T, int N>
-static bool ixfft_pipe_launch(const IxFftArgs<T>& a, cudaStream_t s) {
-    // float only: in double the tiles halve and the k_ixfft_reg form measured faster
-    if constexpr (sizeof(T) != 4) {
-        return false;
-    } else {
-        using P = IPipe<T, N>;
-        if (a.g.NY % P::RB != 0) return false;
-        auto k = k_ixfft_pipe<T, N>;
-        // per size and device (function attributes are per device), resolved at the first launch
-        constexpr int MAXDEV = 64;
-        static int sms_of[MAXDEV] = {}, occ_of[MAXDEV] = {};  // occ 0: not resolved yet, -1: does not fit
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (dev < 0 || dev >= MAXDEV) return false;
-        if (occ_of[dev] == 0) {
-            int optin = 0, o = 0, n = 0;
-            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-            cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-            if (P::smem <= (size_t)optin) {
-                cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::smem);
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k, XP_NT, P::smem);
-            }
-            sms_of[dev] = n;
-            occ_of[dev] = o > 0 ? o : -1;
-        }
-        const int occ = occ_of[dev], sms = sms_of[dev];
-        if (occ < 1) return false;
-        const long long ntile = (long long)(a.g.NY / P::RB) * a.g.NZ;
-        const int grid = (int)std::min<long long>(ntile, (long long)sms * occ);
-        k<<<grid, XP_NT, P::smem, s>>>(a);
-        return true;
-    }
-}
-
 constexpr int DIV_ZC = 4;  // planes per thread of k_div_quad_z
 template <typename T>
 static void div_quad_launch(const DivFftArgs<T>& a, T* out, cudaStream_t s) {
@@ -397,180 +130,66 @@ static void div_quad_launch(const DivFftArgs<T>& a, T* out, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------------------
-// inverse x-FFT
-// ---------------------------------------------------------------------------
-template <typename T, int N>
-__global__ void __launch_bounds__(512) k_ixfft_reg(IxFftArgs<T> a, int rows, int lrows, int alias) {
-    constexpr int N1 = FftSplit<N>::N1, N2 = FftSplit<N>::N2, YL = FftSplit<N>::YL, NH = N / 2, NXH = NH + 1;
-    constexpr int PC = 16 / sizeof(cplx<T>);  // complex values per 16-byte chunk
-    extern __shared__ __align__(16) unsigned char smraw[];
-    const Geom& g = a.g;
-    const int NY = g.NY, nl = rows >> 1, TS = rows + 2;
-    cplx<T>* tile = reinterpret_cast<cplx<T>*>(smraw);  // tile[kx * TS + r]
-    // alias: the first pass's output over the tile itself, every thread holding at most
-    // one line segment (gather all, barrier, transform and write); else after the tile
-    cplx<T>* Y = alias ? tile : tile + NXH * TS;
-    // planes in descending z, the reverse of the inverse y-FFT that wrote them
-    const int z = gridDim.y - 1 - blockIdx.y, y0 = blockIdx.x * rows;
-    {
-        const int cpr = rows / PC, lc = lrows - (PC == 2 ? 1 : 0);
-        for (int e = threadIdx.x; e < NXH * cpr; e += blockDim.x) {
-            const int kx = e >> lc, c = e & (cpr - 1);
-            cp_async<16>(tile + kx * TS + c * PC, a.spec + ((size_t)z * NXH + kx) * NY + y0 + c * PC);
-        }
-        cp_async_commit();
-        cp_async_wait<0>();
-    }
-    __syncthreads();
-    // the Hermitian-extended line of two packed rows at the first pass's positions
-    auto gather = [&](int l, int n2, cplx<T>(&v)[N1]) {
-#pragma unroll
-        for (int n1 = 0; n1 < N1; n1++) {
-            const int k = N2 * n1 + n2;
-            const bool up = k > NH;
-            const cplx<T>* t = tile + (up ? N - k : k) * TS + 2 * l;
-            cplx<T> av = t[0], bv = t[1];
-            if (up) {
-                av.y = -av.y;
-                bv.y = -bv.y;
-            }
-            if (k == 0 || k == NH) {
-                av.y = 0;
-                bv.y = 0;
-            }
-            v[n1] = {av.x - bv.y, av.y + bv.x};
-        }
-    };
-    if (alias) {
-        const bool mine = (int)threadIdx.x < nl * N2;
-        const int l = threadIdx.x / N2, n2 = threadIdx.x - l * N2;
-        cplx<T> v[N1];
-        if (mine) gather(l, n2, v);
-        __syncthreads();
-        if (mine) fft_pass_a<T, N, +1>(v, n2, a.twx, Y + l * YL);
-    } else {
-        for (int it = threadIdx.x; it < nl * N2; it += blockDim.x) {
-            const int l = it / N2, n2 = it - l * N2;
-            cplx<T> v[N1];
-            gather(l, n2, v);
-            fft_pass_a<T, N, +1>(v, n2, a.twx, Y + l * YL);
-        }
-    }
-    __syncthreads();
-    const T sc = a.scale;
-    for (int it = threadIdx.x; it < nl * N1; it += blockDim.x) {
-        const int l = it / N1, k1 = it - l * N1;
-        cplx<T> v[N2];
-        fft_pass_b<T, N, +1>(v, k1, Y + l * YL);
-        T* pa = a.p + ((size_t)z * NY + y0 + 2 * l) * N + k1;
-        T* pb = pa + N;
-#pragma unroll
-        for (int k2 = 0; k2 < N2; k2++) {
-            pa[k2 * N1] = v[k2].x * sc;
-            pb[k2 * N1] = v[k2].y * sc;
-        }
-    }
-}
-
-// Double: one thread per first-pass line segment when that takes at most 512 threads, and
-// the tile and the first pass's output share their buffer, which doubles the rows that
-// fit the shared-memory budget (measured at 384x384x256: 0.139 ms against 0.164 ms).
-// Float keeps 256 threads and separate buffers (0.083 ms against 0.087 ms aliased).
-template <typename T, int N>
-static bool ixfft_alias(int rows) {
-    return sizeof(T) == 8 && (rows / 2) * FftSplit<N>::N2 <= 512;
-}
-template <typename T, int N>
-static int ixfft_threads(int rows) {
-    const int items = (rows / 2) * FftSplit<N>::N2;
-    return ixfft_alias<T, N>(rows) ? std::max(256, (items + 31) / 32 * 32) : 256;
-}
-
-template <typename T, int N>
-static size_t ixfft_reg_smem(int rows) {
-    const size_t tile = (size_t)(N / 2 + 1) * (rows + 2), y = (size_t)(rows / 2) * FftSplit<N>::YL;
-    return (ixfft_alias<T, N>(rows) ? std::max(tile, y) : tile + y) * sizeof(cplx<T>);
-}
-
-template <typename T, int N>
-static void ixfft_reg_launch(const IxFftArgs<T>& a, int rows, cudaStream_t s) {
-    const size_t smem = ixfft_reg_smem<T, N>(rows);
-    int lr = 0;
-    while ((1 << lr) < rows) lr++;
-    auto k = k_ixfft_reg<T, N>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k<<<dim3(a.g.NY / rows, a.g.NZ), ixfft_threads<T, N>(rows), smem, s>>>(a, rows, lr,
-                                                                           ixfft_alias<T, N>(rows) ? 1 : 0);
-}
-
-// ---------------------------------------------------------------------------
 // dispatch on the transform length
 // ---------------------------------------------------------------------------
-// Rows per CTA of the x-FFT kernels: the largest of 32, 16, 8 that divides NY and
-// whose shared memory stays within XFFT_SMEM_PREF (four CTAs per SM: measured faster
-// than two), else within 110 KB (two CTAs per SM); 0 if none.
-constexpr size_t XFFT_SMEM_PREF = 56 * 1024;
-template <typename T, int N>
-static int xfft_reg_rows(int NY, bool inverse) {
-    for (size_t cap : {XFFT_SMEM_PREF, (size_t)110 * 1024})
-        for (int r : {32, 16, 8}) {
-            if (NY % r) continue;
-            const size_t sm = inverse ? ixfft_reg_smem<T, N>(r) : div_xfft_reg_smem<T, N>(r);
-            if (sm <= cap) return r;
-        }
-    return 0;
-}
-
 #define TC_FFT_SIZES(X) X(16) X(24) X(32) X(48) X(64) X(96) X(128) X(192) X(256) X(384) X(512) X(768) X(1024)
+TC_FFT_LENGTHS(s, TC_FFT_SIZES)
+
+// The register transforms of the other 2^a 3^b (k_fft_m.cu, k_fft_l.cu), and of y-counts that
+// no power-of-two tile of rows divides, are not used by the mixed SRK step: its dp/dt is a
+// difference of pressures over tau, which any other rounding of a float transform moves by
+// 1e-4 of itself (k_zsolve.cu keeps its z-solve for the same reason).
+template <typename T>
+static bool fft_keep(const Geom& g) {
+    return sizeof(T) == 4 && g.norm_srk != 0;
+}
 
 template <typename T>
 bool launch_yfft_reg(const YFftArgs<T>& a, cudaStream_t s) {
-    switch (a.g.NY) {
-#define TC_CASE(n)                  \
-    case n:                         \
-        yfft_reg_launch<T, n>(a, s); \
-        return true;
-        TC_FFT_SIZES(TC_CASE)
-#undef TC_CASE
-        default: return false;
+    if (yfft_s<T>(a, s)) return true;
+    return !fft_keep<T>(a.g) && (yfft_m<T>(a, s) || yfft_l<T>(a, s));
+}
+
+template <typename T>
+static bool xfft_any(const DivFftArgs<T>& a, const T* src, cudaStream_t s) {
+    if (fft_keep<T>(a.g)) return a.g.NY % 8 == 0 && xfft_s<T>(a, src, s);
+    return xfft_s<T>(a, src, s) || xfft_m<T>(a, src, s) || xfft_l<T>(a, src, s);
+}
+
+// Whether an x-FFT kernel takes these lines (the vector RHS is put through the divergence
+// only then).
+static bool xfft_has(const Geom& g, bool keep) {
+    if (g.NX > 1024 || g.NY % 6 * (g.NY % 8) != 0) return false;
+    switch (g.NX) {
+#define TC_HAS(n) case n:
+        TC_FFT_SIZES(TC_HAS)
+#undef TC_HAS
+        return !keep || g.NY % 8 == 0;
+        default: return !keep;
     }
 }
 
-// The vector RHS first goes through k_div_quad_z into a.dtmp (needs NX % 4 == 0 and a
-// scratch buffer), then the real field is transformed.
+// The vector RHS first goes through the divergence into a.dtmp (a scratch field), then the
+// real field is transformed.
 template <typename T>
 int launch_div_xfft_reg(const DivFftArgs<T>& a, cudaStream_t s) {
-    const bool vec = a.src_scalar == nullptr;
-    if (vec && (a.dtmp == nullptr || a.g.NX % 4 != 0)) return 0;
-    switch (a.g.NX) {
-#define TC_CASE(n)                                           \
-    case n: {                                                \
-        const int rows = xfft_reg_rows<T, n>(a.g.NY, false); \
-        if (!rows) return 0;                                 \
-        if (vec) div_quad_launch<T>(a, a.dtmp, s);           \
-        xfft_reg_launch<T, n>(a, vec ? a.dtmp : a.src_scalar, rows, s); \
-        return vec ? 2 : 1;                                  \
+    const bool vec = a.src_scalar == nullptr, keep = fft_keep<T>(a.g);
+    if (vec && (a.dtmp == nullptr || (keep && a.g.NX % 4 != 0))) return 0;
+    if (!vec) return xfft_any<T>(a, a.src_scalar, s) ? 1 : 0;
+    if (!xfft_has(a.g, keep)) return 0;
+    if (a.g.NX % 4 == 0) {
+        div_quad_launch<T>(a, a.dtmp, s);
+    } else {
+        const DivArgs<T> d{a.g, a.m, a.v, a.dtmp};
+        launch_divergence<T>(d, s);
     }
-        TC_FFT_SIZES(TC_CASE)
-#undef TC_CASE
-        default: return 0;
-    }
+    return xfft_any<T>(a, a.dtmp, s) ? 2 : 0;
 }
 
 template <typename T>
 bool launch_ixfft_reg(const IxFftArgs<T>& a, cudaStream_t s) {
-    switch (a.g.NX) {
-#define TC_CASE(n)                                          \
-    case n: {                                               \
-        const int rows = xfft_reg_rows<T, n>(a.g.NY, true); \
-        if (!rows) return false;                            \
-        if (!ixfft_pipe_launch<T, n>(a, s)) ixfft_reg_launch<T, n>(a, rows, s); \
-        return true;                                        \
-    }
-        TC_FFT_SIZES(TC_CASE)
-#undef TC_CASE
-        default: return false;
-    }
+    if (fft_keep<T>(a.g)) return a.g.NY % 8 == 0 && ixfft_s<T>(a, s);
+    return ixfft_s<T>(a, s) || ixfft_m<T>(a, s) || ixfft_l<T>(a, s);
 }
 
 // The divergence pass alone (for the plane transforms of k_fft_plane.cu): false when the

@@ -236,10 +236,8 @@ int correct_diag_chunks(const Geom& g);  // xy-CTAs per plane of the fused diagn
 void launch_diag_finish(const double* part, double* planes, int NZ, int S, cudaStream_t s);
 void launch_stats_acc(const double* planes, double* acc, int NZ, double inv_nxy, double w, cudaStream_t s);
 
-// State of a device-controlled run (tc_run_graph): bodies done, their bound, the CFL
-// number of the last check and the bounds that keep the loop going.
 // out[i] = post * (c[0] x[0][i] + c[1] x[1][i] + ... + c[nt-1] x[nt-1][i]), summed left
-// to right in T; x may alias out (elementwise).  The stage updates of the SRK step.
+// to right in T; x may alias out (elementwise).
 constexpr int TC_LIN_MAX = 8;
 template <typename T>
 struct LinComb {
@@ -252,28 +250,34 @@ struct LinComb {
 };
 template <typename T> void launch_lincomb(const LinComb<T>& a, cudaStream_t s);
 
-// Pressure bookkeeping of one SRK stage (collocated_SRK/func_global.h:356-380 and
-// :391-395), one pass each.  rhs (mode 0): muj = c0 x + sum_j cm_j mujt_j with x = p
-// (StabType 0) or dp/dt (1); StabType 1 also pjhat = p + cpd dp/dt + sum_j cq_j qj_j;
-// bufs = muj + pjhat - cb dp/dt (1) or muj - cb p (0).  post (mode 1): pj = mujt_i +
-// bufs; mujt_i -= cb (dp/dt or p); StabType 1 also qj_i = inv (pj - pjhat).
+// One pointwise pass of the SRK step (k_srk.cu).  Vectors are bases of three blocks of N.
+//   field  = ga (+ gb, then ga is the solve's mu);  K = rhs - G field -> kout
+//   vout   = own_first: K + sum_k c_k x_k;  else x_0 + sum_{k>0} c_k x_k + c_own K
+//   nu1    = K + alpha x_0
+// and, with xs = dp/dt (StabType 1) or p (0), after a solve (gb): mu = ga - cb xs -> mu_out,
+// field -> p_out, StabType 1 q = inv (field - pjhat) -> q_out; then the next stage's
+//   pjhat = p (+ cpd xs) + sum_j cq_j q_j (+ cq[nj] q)            (StabType 1)
+//   buf_out = c0 xs + sum_j cm_j mujt_j (+ cm[nj] mu) (+ pjhat) - cb xs
+// Null outputs are skipped; ga null: the scalar part alone.
 template <typename T>
-struct SrkScal {
-    int mode, stab, nj;
-    const T* p;
-    const T* dpdt;
-    const T* mujt[TC_LIN_MAX];
-    const T* qj[TC_LIN_MAX];
-    double c0, cm[TC_LIN_MAX], cq[TC_LIN_MAX], cpd, cb, inv;
-    T* bufs;
-    T* pjhat;
-    T* pj;
-    T* mujt_i;
-    T* qj_i;
-    long long n;
+struct SrkStage {
+    Geom g;
+    MeshDev<T> m;
+    const T *ga = nullptr, *gb = nullptr, *rhs = nullptr;
+    T *kout = nullptr, *vout = nullptr, *nu1 = nullptr;
+    int own_first = 0, nt = 0;
+    const T* x[TC_LIN_MAX];
+    T c[TC_LIN_MAX], c_own = 0, alpha = 0;
+    int stab = 0, nj = 0, use_cpd = 0;
+    const T *xs = nullptr, *p = nullptr;
+    const T *mujt[TC_LIN_MAX], *qj[TC_LIN_MAX];
+    T c0 = 0, cm[TC_LIN_MAX], cq[TC_LIN_MAX], cpd = 0, cb = 0, inv = 0;
+    T *pjhat = nullptr, *mu_out = nullptr, *q_out = nullptr, *p_out = nullptr, *buf_out = nullptr;
 };
-template <typename T> void launch_srk_scal(const SrkScal<T>& a, cudaStream_t s);
+template <typename T> void launch_srk_stage(const SrkStage<T>& a, cudaStream_t s);
 
+// State of a device-controlled run (tc_run_graph): bodies done, their bound, the CFL
+// number of the last check and the bounds that keep the loop going.
 struct RunCtl {
     unsigned iters, max_iters;
     double cfl, cfl_min, cfl_max;

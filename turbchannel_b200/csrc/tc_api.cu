@@ -16,7 +16,6 @@
 #include <mutex>
 #include <random>
 #include <string>
-#include <initializer_list>
 #include <utility>
 #include <vector>
 
@@ -454,6 +453,19 @@ static void fill_flux_plane_consts(const Geom& g, const HostMesh& hm, std::vecto
     }
 }
 
+// Bytes of the z-solve's factor buffers: in the mixed collocated scheme for the step's layout
+// and for the SRK step's.
+static void zfactor_capacity(const Geom& g, int eb, size_t& fac, size_t& low) {
+    fac = zfactor_bytes(g, eb);
+    low = eb == 4 ? zfactor_low_bytes(g) : 0;
+    if (eb == 4 && g.scheme == TC_SCHEME_COLLOC) {
+        Geom q = g;
+        q.norm_srk = 1;
+        fac = std::max(fac, zfactor_bytes(q, eb));
+        low = std::max(low, zfactor_low_bytes(q));
+    }
+}
+
 static int static_zscr(void** out);
 
 extern "C" int tc_create(const tc_params* prm, const double* zz, tc_handle** out) {
@@ -538,8 +550,10 @@ extern "C" int tc_create(const tc_params* prm, const double* zz, tc_handle** out
     if (p.turb_model != TC_TURB_NONE) TC_ALLOC(h->nu_t, N * E);
     TC_ALLOC(h->ptmp, N * E);
     TC_ALLOC(h->spec, (size_t)g.NXH * g.NY * g.NZ * 2 * E);
-    TC_ALLOC(h->zfac, zfactor_bytes(g, (int)E));
-    if (!h->fp64) TC_ALLOC(h->zfac_low, zfactor_low_bytes(g));
+    size_t zf = 0, zl = 0;
+    zfactor_capacity(g, (int)E, zf, zl);
+    TC_ALLOC(h->zfac, zf);
+    if (zl) TC_ALLOC(h->zfac_low, zl);
     // mesh arrays, 9 slots of NZ+2 (the last one holds MAT_A, up to 3 NZ entries), then
     // the per-plane reciprocals (TC_PC per plane) the Smagorinsky factor and the closure's two constants (one per plane each)
     const int L = g.NZ + 2;
@@ -638,8 +652,8 @@ extern "C" int tc_create(const tc_params* prm, const double* zz, tc_handle** out
         cudaMemsetAsync(h->pres[l], 0, N * E, h->st);
     }
     if (h->nu_t) cudaMemsetAsync(h->nu_t, 0, N * E, h->st);
-    cudaMemsetAsync(h->zfac, 0, zfactor_bytes(g, (int)E), h->st);
-    if (h->zfac_low) cudaMemsetAsync(h->zfac_low, 0, zfactor_low_bytes(g), h->st);
+    cudaMemsetAsync(h->zfac, 0, zf, h->st);
+    if (h->zfac_low) cudaMemsetAsync(h->zfac_low, 0, zl, h->st);
     if (h->fp64) {
         ZSolveArgs<double> za{g, mesh_dev<double>(h), mode_tabs(h), (cplx<double>*)h->spec, nullptr, h->err_flag, h->zfac,
                               h->zfac_low};
@@ -1378,150 +1392,150 @@ static size_t srk_bytes(const tc_handle* h, int S, size_t eb) {
     return ((size_t)(S + 2) * 3 + (size_t)2 * S + 3) * (size_t)h->g.N * eb;
 }
 
-template <typename T>
-struct SrkOps {
-    tc_handle* h;
-    void lin(void* out, long long n, std::initializer_list<std::pair<double, const void*>> terms, double post = 1.0) {
-        std::vector<std::pair<double, const void*>> v(terms);
-        lin_v(out, n, v, post);
-    }
-    void lin_v(void* out, long long n, const std::vector<std::pair<double, const void*>>& v, double post = 1.0) {
-        LinComb<T> a{};
-        a.out = (T*)out;
-        a.nt = (int)v.size();
-        for (int k = 0; k < a.nt; k++) {
-            a.c[k] = v[k].first;
-            a.x[k] = (const T*)v[k].second;
-        }
-        a.post = post;
-        a.n = n;
-        launch_lincomb<T>(a, h->st);
-        h->launches += 1;
-    }
-    void explicit_term(const void* v, void* out) {
-        FluxArgs<T> fa{};
-        fa.g = h->g;
-        fa.m = mesh_dev<T>(h);
-        fa.vel = cvec<T>((void*)v, h->g.N);
-        fa.fout = vec<T>(out, h->g.N);
-        fa.nu_t = nullptr;
-        fa.order = 0;
-        launch_flux_coll<T>(fa, h->st);
-        h->launches += 1;
-    }
-    // out = rhs - G p (the correction kernel with tob = 1; out may alias rhs)
-    void grad_sub(const void* rhs, const void* p, void* out) {
-        CorrArgs<T> ca{};
-        ca.g = h->g;
-        ca.m = mesh_dev<T>(h);
-        ca.rhs = cvec<T>((void*)rhs, h->g.N);
-        ca.p = (const T*)p;
-        ca.vout = vec<T>(out, h->g.N);
-        ca.tob = (T)1;
-        launch_correct<T>(ca, h->st);
-        h->launches += 1;
-    }
-};
-
+// The passes and their fusion: k_srk.cu.  Coefficients that are zero in the tables leave
+// their array unread (an exact zero).
 template <typename T>
 static int srk_step_impl(tc_handle* h, double tau) {
     const auto& s = h->srk;
     const int S = s.S;
-    const long long N = h->g.N, N3 = 3 * N;
+    const long long N = h->g.N;
     const SrkBufs b = srk_bufs(h, sizeof(T));
-    auto KH = [&](int j) { return (void*)(b.kuhat + j * b.vb); };
-    auto MT = [&](int j) { return (void*)(b.mujt + j * b.sb); };
-    auto QJ = [&](int j) { return (void*)(b.qj + j * b.sb); };
-    void* vel = h->vel[0];
-    void* pres = h->pres[0];
-    void* dpdt = h->pres[1];
+    auto KH = [&](int j) { return (T*)(b.kuhat + j * b.vb); };
+    auto MT = [&](int j) { return (T*)(b.mujt + j * b.sb); };
+    auto QJ = [&](int j) { return (T*)(b.qj + j * b.sb); };
+    T *vel = (T*)h->vel[0], *pres = (T*)h->pres[0], *dpdt = (T*)h->pres[1], *bufv = (T*)b.bufv;
     const double ass = s.BI[S * S - 1], inv_ass = 1. / ass, tau_stage = tau * ass, inv_tau_stage = 1. / tau_stage;
     const double alpha = s.alpha_tau / tau;
     const bool ck = s.type == TC_IMEX_CK, atype = s.type == TC_IMEX_A;
-    SrkOps<T> op{h};
-    if (!atype) {  // func_global.h:324-328
-        op.explicit_term(vel, KH(0));
-        op.grad_sub(KH(0), pres, KH(0));
-    }
-    if (ck) op.lin(b.nu1, N3, {{1.0, KH(0)}, {alpha, vel}});  // func_global.h:329-332
     const int j0 = atype ? 0 : 1;
-    std::vector<std::pair<double, const void*>> t;
-    for (int i = j0; i < S; i++) {
-        // stage velocity u = u_n + tau sum_j aE_ij Kuhat_j (func_global.h:340-347)
-        t.assign({{1.0, vel}});
-        for (int j = 0; j < i; j++) t.push_back({tau * s.BE[i * S + j], KH(j)});
-        op.lin_v(b.bufv, N3, t);
-        op.explicit_term(b.bufv, KH(i));
-        // right-hand side of the pressure system (func_global.h:356-380), one pass
+    // the pass reads one buf around each node and writes the next stage's: two buffers, the
+    // second in the last stage's unused mu
+    T *buf = (T*)b.bufs, *buf2 = MT(S - 1);
+    auto explicit_term = [&](const T* v, T* out) {
+        FluxArgs<T> fa{};
+        fa.g = h->g;
+        fa.m = mesh_dev<T>(h);
+        fa.vel = cvec<T>((void*)v, N);
+        fa.fout = vec<T>(out, N);
+        fa.order = 0;
+        launch_flux_coll<T>(fa, h->st);
+        h->launches += 1;
+    };
+    auto pass = [&]() {
+        SrkStage<T> a;
+        a.g = h->g;
+        a.m = mesh_dev<T>(h);
+        a.stab = s.stab;
+        a.cb = (T)(s.stab ? alpha * tau_stage * tau_stage : alpha * tau_stage);
+        return a;
+    };
+    auto run = [&](const SrkStage<T>& a) {
+        launch_srk_stage<T>(a, h->st);
+        h->launches += 1;
+    };
+    // velocity of stage `row` (the step's result for row S) from the K of stages below `own`
+    // and the pass's own one (func_global.h:340-347, :400-407)
+    auto velocity = [&](SrkStage<T>& a, int row, int own, T* out) {
+        a.vout = out;
+        a.nt = 0;
+        a.x[a.nt] = vel;
+        a.c[a.nt++] = (T)1;
+        for (int j = 0; j < own; j++)
+            if (s.BE[row * S + j] != 0.0) {
+                a.x[a.nt] = KH(j);
+                a.c[a.nt++] = (T)(tau * s.BE[row * S + j]);
+            }
+        a.c_own = (T)(tau * s.BE[row * S + own]);
+    };
+    // right-hand side of stage i's pressure system (func_global.h:356-380)
+    auto next_buf = [&](SrkStage<T>& a, int i, T* out) {
         const double ck0 = ck ? (1. - s.alpha_tau * s.BI[i * S]) : 1.0;
-        SrkScal<T> sc{};
-        sc.stab = s.stab;
-        sc.p = (const T*)pres;
-        sc.dpdt = (const T*)dpdt;
-        sc.n = N;
-        sc.bufs = (T*)b.bufs;
-        sc.pjhat = (T*)b.pjhat;
-        sc.mode = 0;
-        sc.nj = i - j0;
+        a.xs = s.stab ? dpdt : pres;
+        a.p = pres;
+        a.c0 = (T)(s.stab ? tau_stage * ck0 : ck0);
+        a.cpd = (T)(tau * s.BI[i * S]);
+        a.use_cpd = s.stab && ck && tau * s.BI[i * S] != 0.0;
+        a.nj = std::max(0, i - 1 - j0);
         for (int j = j0; j < i; j++) {
-            sc.mujt[j - j0] = (const T*)MT(j);
-            sc.qj[j - j0] = (const T*)QJ(j);
-            sc.cm[j - j0] = inv_ass * s.BI[i * S + j];
-            sc.cq[j - j0] = tau * s.BI[i * S + j];
+            a.mujt[j - j0] = MT(j);
+            a.qj[j - j0] = QJ(j);
+            a.cm[j - j0] = (T)(inv_ass * s.BI[i * S + j]);
+            a.cq[j - j0] = (T)(tau * s.BI[i * S + j]);
         }
-        sc.c0 = s.stab ? tau_stage * ck0 : ck0;
-        sc.cpd = (s.stab && ck) ? tau * s.BI[i * S] : 0.0;
-        sc.cb = s.stab ? alpha * tau_stage * tau_stage : alpha * tau_stage;
-        launch_srk_scal<T>(sc, h->st);
-        h->launches += 1;
-        op.grad_sub(KH(i), b.bufs, b.bufv);  // func_global.h:381-386
-        t.assign({{1.0, b.bufv}, {alpha, vel}});
-        if (ck) t.push_back({-s.d[i], b.nu1});
-        op.lin_v(b.bufv, N3, t);
-        poisson<T>(h, b.bufv, nullptr, MT(i));  // UnapplyGradient
-        sc.mode = 1;  // func_global.h:391-395: pj, mujt_i, qj_i in one pass
-        sc.pj = (T*)b.pj;
-        sc.mujt_i = (T*)MT(i);
-        sc.qj_i = (T*)QJ(i);
-        sc.inv = inv_tau_stage;
-        launch_srk_scal<T>(sc, h->st);
-        h->launches += 1;
-        op.grad_sub(KH(i), b.pj, KH(i));
+        a.pjhat = (T*)b.pjhat;
+        a.buf_out = out;
+    };
+    {
+        SrkStage<T> a = pass();
+        if (!atype) {  // func_global.h:324-332
+            explicit_term(vel, KH(0));
+            a.rhs = KH(0);
+            a.ga = pres;
+            a.kout = KH(0);
+            velocity(a, 1, 0, S == 1 ? vel : bufv);
+            if (ck) {
+                a.nu1 = (T*)b.nu1;
+                a.alpha = (T)alpha;
+            }
+        }
+        if (j0 < S) next_buf(a, j0, buf);
+        run(a);
     }
-    // final solution (func_global.h:400-407)
-    t.assign({{1.0, vel}});
-    for (int j = 0; j < S; j++) t.push_back({tau * s.BE[S * S + j], KH(j)});
-    op.lin_v(vel, N3, t);
-    TC_CUDA(cudaMemcpyAsync(pres, b.pj, b.sb, cudaMemcpyDeviceToDevice, h->st));
-    if (s.stab) TC_CUDA(cudaMemcpyAsync(dpdt, QJ(S - 1), b.sb, cudaMemcpyDeviceToDevice, h->st));
+    if (j0 >= S) {  // an explicit single stage has no pressure system
+        TC_CUDA(cudaMemsetAsync(pres, 0, b.sb, h->st));
+        if (s.stab) TC_CUDA(cudaMemsetAsync(dpdt, 0, b.sb, h->st));
+    }
+    for (int i = j0; i < S; i++) {
+        const bool last = i == S - 1;
+        explicit_term(i == 0 ? vel : bufv, KH(i));
+        {  // func_global.h:381-386
+            SrkStage<T> a = pass();
+            a.rhs = KH(i);
+            a.ga = buf;
+            a.vout = bufv;
+            a.own_first = 1;
+            a.x[0] = vel;
+            a.c[0] = (T)alpha;
+            a.nt = 1;
+            if (ck) {
+                a.x[1] = (const T*)b.nu1;
+                a.c[1] = (T)(-s.d[i]);
+                a.nt = 2;
+            }
+            run(a);
+        }
+        poisson<T>(h, bufv, nullptr, b.pj);  // UnapplyGradient
+        SrkStage<T> a = pass();  // func_global.h:391-395
+        a.rhs = KH(i);
+        a.ga = (const T*)b.pj;
+        a.gb = buf;
+        a.kout = last ? nullptr : KH(i);
+        velocity(a, last ? S : i + 1, i, last ? vel : bufv);
+        if (last) {
+            a.xs = s.stab ? dpdt : pres;
+            a.pjhat = (T*)b.pjhat;
+        } else {
+            next_buf(a, i + 1, buf2);
+            a.mu_out = MT(i);
+        }
+        a.inv = (T)inv_tau_stage;
+        if (s.stab) a.q_out = last ? dpdt : QJ(i);
+        a.p_out = last ? pres : nullptr;
+        run(a);
+        std::swap(buf, buf2);
+    }
     h->fused_valid = false;
     return check_launch("tc_srk_step");
 }
 
 static void run_graph_drop(tc_handle* h);
 
-// The mixed SRK step solves its banded systems from factors of its own layout: rebuilt once,
-// when the handle becomes an SRK one.
+// The mixed SRK step solves its banded systems from factors of its own layout: written over
+// the step's (the buffers hold either, zfactor_capacity) when the handle becomes an SRK one.
 static int srk_refactor(tc_handle* h) {
     TC_CUDA(cudaStreamSynchronize(h->st));
-    run_graph_drop(h);  // a captured run holds the old factors
-    const Geom& g = h->g;
-    const size_t nf = zfactor_bytes(g, (int)h->esz), nl = zfactor_low_bytes(g);
-    void *f = nullptr, *fl = nullptr;
-    if (cudaMalloc(&f, nf) != cudaSuccess || cudaMalloc(&fl, nl) != cudaSuccess) {
-        cudaGetLastError();
-        if (f) cudaFree(f);
-        h->srk.S = 0;
-        h->g.norm_srk = 0;  // the handle keeps its factors
-        return fail(TC_E_NOMEM, "tc_srk_init: z-solve factors");
-    }
-    cudaFree(h->zfac);
-    cudaFree(h->zfac_low);
-    h->zfac = f;
-    h->zfac_low = fl;
-    TC_CUDA(cudaMemsetAsync(f, 0, nf, h->st));
-    TC_CUDA(cudaMemsetAsync(fl, 0, nl, h->st));
-    ZSolveArgs<float> za{g, mesh_dev<float>(h), mode_tabs(h), (cplx<float>*)h->spec, nullptr, h->err_flag, h->zfac,
+    run_graph_drop(h);  // a captured run solves from the other layout
+    ZSolveArgs<float> za{h->g, mesh_dev<float>(h), mode_tabs(h), (cplx<float>*)h->spec, nullptr, h->err_flag, h->zfac,
                          h->zfac_low};
     launch_zfactor<float>(za, h->st);
     return check_launch("tc_srk_init");

@@ -24,6 +24,8 @@ namespace tc {
 template <typename T, int SCHEME, int ZC>
 __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 3 : 4) k_div_quad_z(DivFftArgs<T> a, T* __restrict__ out) {
     const Geom& g = a.g;
+    pdl_launch();
+    pdl_wait();
     const int NX = g.NX, NY = g.NY, NZ = g.NZ, NQ = NX >> 2, NZB = (NZ + ZC - 1) / ZC;
     const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= (long long)NQ * NY * NZB) return;
@@ -124,9 +126,9 @@ template <typename T>
 static void div_quad_launch(const DivFftArgs<T>& a, T* out, cudaStream_t s) {
     const long long nq = (long long)(a.g.NX / 4) * a.g.NY * ((a.g.NZ + DIV_ZC - 1) / DIV_ZC);
     const unsigned nb = (unsigned)((nq + 255) / 256);
-    if (a.g.scheme == TC_SCHEME_VV4) k_div_quad_z<T, TC_SCHEME_VV4, DIV_ZC><<<nb, 256, 0, s>>>(a, out);
-    else if (a.g.scheme == TC_SCHEME_HW2) k_div_quad_z<T, TC_SCHEME_HW2, DIV_ZC><<<nb, 256, 0, s>>>(a, out);
-    else k_div_quad_z<T, TC_SCHEME_COLLOC, DIV_ZC><<<nb, 256, 0, s>>>(a, out);
+    if (a.g.scheme == TC_SCHEME_VV4) launch_pdl(a.g.pdl, k_div_quad_z<T, TC_SCHEME_VV4, DIV_ZC>, nb, 256, 0, s, a, out);
+    else if (a.g.scheme == TC_SCHEME_HW2) launch_pdl(a.g.pdl, k_div_quad_z<T, TC_SCHEME_HW2, DIV_ZC>, nb, 256, 0, s, a, out);
+    else launch_pdl(a.g.pdl, k_div_quad_z<T, TC_SCHEME_COLLOC, DIV_ZC>, nb, 256, 0, s, a, out);
 }
 
 // ---------------------------------------------------------------------------

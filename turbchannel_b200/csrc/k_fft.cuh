@@ -35,6 +35,8 @@ __global__ void __launch_bounds__(256) k_yfft_reg(cplx<T>* spec, long long nline
     constexpr int LINES = yfft_reg_lines<T, N>();
     extern __shared__ __align__(16) unsigned char smraw[];
     cplx<T>* Y = reinterpret_cast<cplx<T>*>(smraw);
+    pdl_launch();
+    pdl_wait();
     // the forward transform takes the lines in descending z, the reverse of the x-FFT that
     // wrote them (its last planes are still in L2), and leaves the low planes, which the
     // z-solve's forward sweep reads first, written last (384x256x384 float: y-FFT 0.052
@@ -68,8 +70,8 @@ static void yfft_reg_launch(const YFftArgs<T>& a, cudaStream_t s) {
     const long long total = (long long)a.g.NZ * a.g.NXH;
     const size_t smem = (size_t)LINES * FftSplit<N>::YL * sizeof(cplx<T>);
     auto k = a.sign < 0 ? k_yfft_reg<T, N, -1> : k_yfft_reg<T, N, +1>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k<<<(unsigned)((total + LINES - 1) / LINES), 256, smem, s>>>(a.spec, total, a.twy);
+    smem_limit(k, smem);
+    launch_pdl(a.g.pdl, k, (unsigned)((total + LINES - 1) / LINES), 256, smem, s, a.spec, total, a.twy);
 }
 
 // ---------------------------------------------------------------------------
@@ -91,6 +93,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_xfft_reg(DivFft
     constexpr int N1 = FftSplit<N>::N1, N2 = FftSplit<N>::N2, YL = FftSplit<N>::YL, ZS = N + 1;
     extern __shared__ __align__(16) unsigned char smraw[];
     const Geom& g = a.g;
+    pdl_launch();
+    pdl_wait();
     const int NY = g.NY, NXH = N / 2 + 1, nl = rows >> 1;
     cplx<T>* Y = reinterpret_cast<cplx<T>*>(smraw);
     // transformed lines, stride N+1: over Y itself when every thread holds at most one
@@ -150,8 +154,8 @@ template <typename T, int N>
 static void xfft_reg_launch(const DivFftArgs<T>& a, const T* src, int rows, cudaStream_t s) {
     const size_t smem = div_xfft_reg_smem<T, N>(rows);
     auto k = k_xfft_reg<T, N>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k<<<dim3(a.g.NY / rows, a.g.NZ), 256, smem, s>>>(a, src, rows, fft_magic(rows));
+    smem_limit(k, smem);
+    launch_pdl(a.g.pdl, k, dim3(a.g.NY / rows, a.g.NZ), 256, smem, s, a, src, rows, fft_magic(rows));
 }
 
 // ---------------------------------------------------------------------------
@@ -181,6 +185,8 @@ __global__ void __launch_bounds__(XP_NT) k_ixfft_pipe(IxFftArgs<T> a) {
     const Geom& g = a.g;
     const int NY = g.NY, YB = NY / RB;
     const long long ntile = (long long)YB * g.NZ;
+    pdl_launch();
+    pdl_wait();
     // tiles in ascending z: the correction that reads p next walks the planes downwards,
     // so that the next step's flux kernel, which starts at z = 0, finds the low planes of
     // the new velocity in L2 (at 384x256x384 the flux kernel gains more, 7 us, than this
@@ -272,7 +278,7 @@ static bool ixfft_pipe_launch(const IxFftArgs<T>& a, cudaStream_t s) {
         if (occ < 1) return false;
         const long long ntile = (long long)(a.g.NY / P::RB) * a.g.NZ;
         const int grid = (int)std::min<long long>(ntile, (long long)sms * occ);
-        k<<<grid, XP_NT, P::smem, s>>>(a);
+        launch_pdl(a.g.pdl, k, grid, XP_NT, P::smem, s, a);
         return true;
     }
 }
@@ -286,6 +292,8 @@ __global__ void __launch_bounds__(512) k_ixfft_reg(IxFftArgs<T> a, int rows, uns
     constexpr int PC = 16 / sizeof(cplx<T>);  // complex values per 16-byte chunk
     extern __shared__ __align__(16) unsigned char smraw[];
     const Geom& g = a.g;
+    pdl_launch();
+    pdl_wait();
     const int NY = g.NY, nl = rows >> 1, TS = rows + 2;
     cplx<T>* tile = reinterpret_cast<cplx<T>*>(smraw);  // tile[kx * TS + r]
     // alias: the first pass's output over the tile itself, every thread holding at most
@@ -377,9 +385,8 @@ template <typename T, int N>
 static void ixfft_reg_launch(const IxFftArgs<T>& a, int rows, cudaStream_t s) {
     const size_t smem = ixfft_reg_smem<T, N>(rows);
     auto k = k_ixfft_reg<T, N>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k<<<dim3(a.g.NY / rows, a.g.NZ), ixfft_threads<T, N>(rows), smem, s>>>(
-        a, rows, fft_magic(rows / (16 / (int)sizeof(cplx<T>))), ixfft_alias<T, N>(rows) ? 1 : 0);
+    smem_limit(k, smem);
+    launch_pdl(a.g.pdl, k, dim3(a.g.NY / rows, a.g.NZ), ixfft_threads<T, N>(rows), smem, s, a, rows, fft_magic(rows / (16 / (int)sizeof(cplx<T>))), ixfft_alias<T, N>(rows) ? 1 : 0);
 }
 
 // Rows per CTA of the x-FFT kernels: the largest of 32, 16, 8 (NY = 2 or 4 times a power of

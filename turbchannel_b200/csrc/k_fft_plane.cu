@@ -72,6 +72,8 @@ __global__ void __launch_bounds__(PF_NT) k_xyfft_plane(const T* __restrict__ src
     cplx<T>* Y = reinterpret_cast<cplx<T>*>(smraw + P::tile_bytes);
     cg::cluster_group cl = cg::this_cluster();
     const int r = (int)cl.block_rank(), z = blockIdx.x / CS, tid = threadIdx.x;
+    pdl_launch();
+    pdl_wait();
 
     // x-FFT of rows r*RY .. r*RY+RY-1, BR at a time, into tile[kx][y - r*RY]
     const T* rows = src + ((size_t)z * NY + (size_t)r * RY) * NX;
@@ -154,6 +156,8 @@ __global__ void __launch_bounds__(PF_NT) k_ixyfft_plane(const cplx<T>* __restric
     cplx<T>* Y = reinterpret_cast<cplx<T>*>(smraw + P::tile_bytes);
     cg::cluster_group cl = cg::this_cluster();
     const int r = (int)cl.block_rank(), z = blockIdx.x / CS, tid = threadIdx.x;
+    pdl_launch();
+    pdl_wait();
     // every CTA of the cluster has started (its shared memory exists) before the first
     // remote store; the arrive is issued now and waited on just before those stores
     asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
@@ -236,7 +240,8 @@ __global__ void __launch_bounds__(PF_NT) k_ixyfft_plane(const cplx<T>* __restric
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-static cudaLaunchConfig_t plane_config(cudaLaunchAttribute* at, int nz, size_t smem, cudaStream_t s) {
+// at: two attributes, the cluster shape and the programmatic launch
+static cudaLaunchConfig_t plane_config(cudaLaunchAttribute* at, bool pdl, int nz, size_t smem, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(PF_CS * nz));
     cfg.blockDim = dim3(PF_NT);
@@ -246,8 +251,10 @@ static cudaLaunchConfig_t plane_config(cudaLaunchAttribute* at, int nz, size_t s
     at->val.clusterDim.x = PF_CS;
     at->val.clusterDim.y = 1;
     at->val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = pdl ? 2 : 1;
     return cfg;
 }
 
@@ -257,8 +264,8 @@ static bool cluster_fits(const void* k, size_t smem) {
         cudaGetLastError();
         return false;
     }
-    cudaLaunchAttribute at;
-    const cudaLaunchConfig_t cfg = plane_config(&at, 1, smem, 0);
+    cudaLaunchAttribute at[2];
+    const cudaLaunchConfig_t cfg = plane_config(at, false, 1, smem, 0);
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
         cudaGetLastError();
@@ -290,22 +297,22 @@ static bool plane_fits() {
 }
 
 template <typename T, int NX, int NY>
-static void plane_fwd(const T* src, cplx<T>* spec, const cplx<T>* twx, const cplx<T>* twy, int nz, cudaStream_t s) {
+static void plane_fwd(const T* src, cplx<T>* spec, const cplx<T>* twx, const cplx<T>* twy, bool pdl, int nz, cudaStream_t s) {
     using P = PlaneFft<T, NX, NY>;
     if constexpr (P::ok) {
-        cudaLaunchAttribute at;
-        const cudaLaunchConfig_t cfg = plane_config(&at, nz, P::smem, s);
+        cudaLaunchAttribute at[2];
+        const cudaLaunchConfig_t cfg = plane_config(at, pdl, nz, P::smem, s);
         cudaLaunchKernelEx(&cfg, k_xyfft_plane<T, NX, NY>, src, spec, twx, twy);
     }
 }
 
 template <typename T, int NX, int NY>
-static void plane_inv(const cplx<T>* spec, T* p, const cplx<T>* twx, const cplx<T>* twy, T scale, int nz,
+static void plane_inv(const cplx<T>* spec, T* p, const cplx<T>* twx, const cplx<T>* twy, T scale, bool pdl, int nz,
                       cudaStream_t s) {
     using P = PlaneFft<T, NX, NY>;
     if constexpr (P::ok) {
-        cudaLaunchAttribute at;
-        const cudaLaunchConfig_t cfg = plane_config(&at, nz, P::smem, s);
+        cudaLaunchAttribute at[2];
+        const cudaLaunchConfig_t cfg = plane_config(at, pdl, nz, P::smem, s);
         cudaLaunchKernelEx(&cfg, k_ixyfft_plane<T, NX, NY>, spec, p, twx, twy, scale);
     }
 }
@@ -332,7 +339,7 @@ int launch_div_xyfft_plane(const DivFftArgs<T>& a, const cplx<T>* twy, cudaStrea
     const T* src = vec ? a.dtmp : a.src_scalar;
 #define TC_CASE(x, y)                                              \
     if (a.g.NX == x && a.g.NY == y) {                              \
-        plane_fwd<T, x, y>(src, a.spec, a.twx, twy, a.g.NZ, s);   \
+        plane_fwd<T, x, y>(src, a.spec, a.twx, twy, a.g.pdl, a.g.NZ, s); \
         return vec ? 2 : 1;                                        \
     }
     TC_PLANE_SIZES(TC_CASE)
@@ -345,7 +352,7 @@ bool launch_ixyfft_plane(const IxFftArgs<T>& a, const cplx<T>* twy, cudaStream_t
     if (!plane_fft_ok<T>(a.g)) return false;
 #define TC_CASE(x, y)                                                        \
     if (a.g.NX == x && a.g.NY == y) {                                        \
-        plane_inv<T, x, y>(a.spec, a.p, a.twx, twy, a.scale, a.g.NZ, s);     \
+        plane_inv<T, x, y>(a.spec, a.p, a.twx, twy, a.scale, a.g.pdl, a.g.NZ, s); \
         return true;                                                         \
     }
     TC_PLANE_SIZES(TC_CASE)

@@ -86,6 +86,8 @@ __device__ __forceinline__ void visc_galerkin(const ACC& A, const NUT& nut, int 
 // CY: nodes per thread along y (the tile is 32 x 8 CY nodes): two for float, one for double.
 template <typename T, int VISC, bool LES, int ORDER, bool STAB1, bool VEC, int CY>
 __global__ void __launch_bounds__(STX* STY, 2) k_flux_coll(FluxArgs<T> a, int tz) {
+    pdl_launch();
+    pdl_wait();
     using ACC = RingAcc<T, 1, CY>;
     constexpr int RS = ACC::RS;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -262,11 +264,11 @@ static void run(const FluxArgs<T>& a, cudaStream_t s) {
     constexpr size_t smem = sizeof(T) * 4 * 3 * RingAcc<T, 1, CY>::PL;
     const bool vec = a.g.NX % (16 / (int)sizeof(T)) == 0;
     auto kern = vec ? k_flux_coll<T, VISC, LES, ORDER, STAB1, true, CY> : k_flux_coll<T, VISC, LES, ORDER, STAB1, false, CY>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    smem_limit(kern, smem);
     dim3 grid;
     int tz;
     flux_coll_shape(a.g, CY, grid, tz);
-    kern<<<grid, STX * STY, smem, s>>>(a, tz);
+    launch_pdl(a.g.pdl, kern, grid, STX * STY, smem, s, a, tz);
 }
 
 template <typename T, int VISC, bool LES>

@@ -119,6 +119,8 @@ __device__ __forceinline__ F2 vfma(F2 a, F2 b, F2 c) { return fma2(a, b, c); }
 template <int SCHEME, int ORDER, int RY, bool TMA>
 __global__ void __launch_bounds__(PTX * PTR / RY, 2)
     k_flux_pair(FluxArgs<float> a, int tz, int tmode, int bid_off, int nb_total, const __grid_constant__ CUtensorMap tmap) {
+    pdl_launch();
+    pdl_wait();
     constexpr int H = SCHEME == TC_SCHEME_VV4 ? 3 : 1;
     constexpr int NT = PTX * PTR / RY;
     using ACC = RingX2<H>;
@@ -388,14 +390,14 @@ static void run_pair(const FluxArgs<float>& a, cudaStream_t s) {
     const bool tma = a.staging == 1 && a.g.NX % PCX == 0 && a.g.NY % PTR == 0 && ntx >= 3 && nty >= 3 &&
                      velocity_tensor_map<H>(a, &tm);
     if (!tma) {
-        plain<<<dim3(ntx, nty, nzc), PTX * PTR / PAIR_RY, smem, s>>>(a, tz, 0, 0, tiles * nzc, tm);
+        launch_pdl(a.g.pdl, plain, dim3(ntx, nty, nzc), PTX * PTR / PAIR_RY, smem, s, a, tz, 0, 0, tiles * nzc, tm);
         return;
     }
     auto boxed = k_flux_pair<SCHEME, ORDER, PAIR_RY, true>;
     cudaFuncSetAttribute(boxed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const int ni = (ntx - 2) * (nty - 2) * nzc;
-    boxed<<<dim3(ntx - 2, nty - 2, nzc), PTX * PTR / PAIR_RY, smem, s>>>(a, tz, 1, 0, tiles * nzc, tm);
-    plain<<<dim3(2 * ntx + 2 * (nty - 2), 1, nzc), PTX * PTR / PAIR_RY, smem, s>>>(a, tz, 2, ni, tiles * nzc, tm);
+    launch_pdl(a.g.pdl, boxed, dim3(ntx - 2, nty - 2, nzc), PTX * PTR / PAIR_RY, smem, s, a, tz, 1, 0, tiles * nzc, tm);
+    launch_pdl(a.g.pdl, plain, dim3(2 * ntx + 2 * (nty - 2), 1, nzc), PTX * PTR / PAIR_RY, smem, s, a, tz, 2, ni, tiles * nzc, tm);
 }
 
 template <int SCHEME>

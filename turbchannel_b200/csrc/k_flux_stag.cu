@@ -47,6 +47,8 @@ __device__ __forceinline__ void flux_cell(const RingAcc<T, SCHEME == TC_SCHEME_V
 
 template <typename T, int SCHEME, int VISC, bool LES, int ORDER, bool VEC, int CY, int TY>
 __global__ void __launch_bounds__(STX* TY, 2) k_flux_stag(FluxArgs<T> a, int tz) {
+    pdl_launch();
+    pdl_wait();
     constexpr int H = SCHEME == TC_SCHEME_VV4 ? 3 : 1;
     using ACC = RingAcc<T, H, CY, TY>;
     constexpr int RS = ACC::RS;
@@ -203,11 +205,11 @@ static void run(const FluxArgs<T>& a, cudaStream_t s) {
     const bool vec = a.g.NX % (16 / (int)sizeof(T)) == 0;
     auto kern = vec ? k_flux_stag<T, SCHEME, VISC, LES, ORDER, true, CY, TY>
                     : k_flux_stag<T, SCHEME, VISC, LES, ORDER, false, CY, TY>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    smem_limit(kern, smem);
     dim3 grid;
     int tz;
     flux_stag_shape(a.g, TY * CY, grid, tz);
-    kern<<<grid, STX * TY, smem, s>>>(a, tz);
+    launch_pdl(a.g.pdl, kern, grid, STX * TY, smem, s, a, tz);
 }
 
 template <typename T, int SCHEME, int VISC, bool LES>

@@ -181,6 +181,8 @@ __global__ void __launch_bounds__(128, 4) k_turb_mlp(TurbArgs<T> a, const float*
     __shared__ MlpSmem S;
     __shared__ __align__(16) __nv_bfloat16 Xb[4][32][8];
     mlp_load_smem(S, P);
+    pdl_launch();
+    pdl_wait();
     __syncthreads();
     const Geom& g = a.g;
     const int NX = g.NX, NY = g.NY, NZ = g.NZ;
@@ -273,8 +275,8 @@ template <typename T>
 void launch_turb_mlp(const TurbArgs<T>& a, const float* P, cudaStream_t s) {
     const long long ngrp = (a.g.N + 31) / 32;
     const int nb = (int)std::max<long long>(1, std::min<long long>((ngrp + 3) / 4, 148 * 4));  // one wave
-    if (a.g.scheme == TC_SCHEME_COLLOC) k_turb_mlp<T, true><<<nb, 128, 0, s>>>(a, P);
-    else k_turb_mlp<T, false><<<nb, 128, 0, s>>>(a, P);
+    if (a.g.scheme == TC_SCHEME_COLLOC) launch_pdl(a.g.pdl, k_turb_mlp<T, true>, nb, 128, 0, s, a, P);
+    else launch_pdl(a.g.pdl, k_turb_mlp<T, false>, nb, 128, 0, s, a, P);
 }
 
 template void launch_les_filter<double>(const double*, const double*, const double*, const double*, const double*,

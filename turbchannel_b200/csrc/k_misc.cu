@@ -55,6 +55,8 @@ constexpr int ZC = 4;
 template <typename T, int SCHEME, bool STAB1, bool GRADONLY>
 __global__ void __launch_bounds__(KX* KY) k_correct(CorrArgs<T> a, int tz) {
     const Geom& g = a.g;
+    pdl_launch();
+    pdl_wait();
     const int NX = g.NX, NY = g.NY, NZ = g.NZ;
     const size_t NXY = (size_t)NX * NY;
     const int ix = blockIdx.x * KX + threadIdx.x % KX, iy = blockIdx.y * KY + threadIdx.x / KX;
@@ -141,6 +143,8 @@ template <typename T, int SCHEME, bool STAB1>
 __global__ void __launch_bounds__(QX* QY, 3) k_correct_quad(CorrArgs<T> a) {
     constexpr int ZN = correct_quad_planes<T>();
     const Geom& g = a.g;
+    pdl_launch();
+    pdl_wait();
     const int NX = g.NX, NY = g.NY, NZ = g.NZ, NQ = NX >> 2;
     const size_t NXY = (size_t)NX * NY;
     const int xq = blockIdx.x * QX + threadIdx.x % QX, iy = blockIdx.y * QY + threadIdx.x / QX;
@@ -233,16 +237,16 @@ static void correct_scheme(const CorrArgs<T>& a, cudaStream_t s) {
     if (!a.grad_only && a.g.NX % 4 == 0) {
         constexpr int ZN = correct_quad_planes<T>();
         const dim3 gq((a.g.NX / 4 + QX - 1) / QX, (a.g.NY + QY - 1) / QY, (a.g.NZ + ZN - 1) / ZN);
-        if (a.pnext) k_correct_quad<T, SCHEME, true><<<gq, QX * QY, 0, s>>>(a);
-        else k_correct_quad<T, SCHEME, false><<<gq, QX * QY, 0, s>>>(a);
+        if (a.pnext) launch_pdl(a.g.pdl, k_correct_quad<T, SCHEME, true>, gq, QX * QY, 0, s, a);
+        else launch_pdl(a.g.pdl, k_correct_quad<T, SCHEME, false>, gq, QX * QY, 0, s, a);
         return;
     }
     dim3 grid;
     int tz;
     column_shape(a.g, grid, tz);
-    if (a.grad_only) k_correct<T, SCHEME, false, true><<<grid, KX * KY, 0, s>>>(a, tz);
-    else if (a.pnext) k_correct<T, SCHEME, true, false><<<grid, KX * KY, 0, s>>>(a, tz);
-    else k_correct<T, SCHEME, false, false><<<grid, KX * KY, 0, s>>>(a, tz);
+    if (a.grad_only) launch_pdl(a.g.pdl, k_correct<T, SCHEME, false, true>, grid, KX * KY, 0, s, a, tz);
+    else if (a.pnext) launch_pdl(a.g.pdl, k_correct<T, SCHEME, true, false>, grid, KX * KY, 0, s, a, tz);
+    else launch_pdl(a.g.pdl, k_correct<T, SCHEME, false, false>, grid, KX * KY, 0, s, a, tz);
 }
 
 template <typename T>
@@ -287,6 +291,8 @@ struct GAcc {
 template <typename T>
 __global__ void __launch_bounds__(KX* KY) k_turb_stag(TurbArgs<T> a) {
     const Geom& g = a.g;
+    pdl_launch();
+    pdl_wait();
     const int ix = blockIdx.x * KX + threadIdx.x % KX, iy = blockIdx.y * KY + threadIdx.x / KX, iz = blockIdx.z;
     if (ix >= g.NX || iy >= g.NY) return;
     GAcc<T> A;
@@ -300,6 +306,8 @@ __global__ void __launch_bounds__(KX* KY) k_turb_stag(TurbArgs<T> a) {
 template <typename T>
 __global__ void __launch_bounds__(KX* KY) k_turb_coll(TurbArgs<T> a) {
     const Geom& g = a.g;
+    pdl_launch();
+    pdl_wait();
     const int ix = blockIdx.x * KX + threadIdx.x % KX, iy = blockIdx.y * KY + threadIdx.x / KX, iz = blockIdx.z;
     if (ix >= g.NX || iy >= g.NY) return;
     GAcc<T> A;
@@ -328,8 +336,8 @@ void launch_turb(const TurbArgs<T>& a, cudaStream_t s) {
     const bool coll = a.g.scheme == TC_SCHEME_COLLOC;
     // collocated: the NZ-1 element layers between the node planes (the top plane keeps its value)
     const dim3 grid((a.g.NX + KX - 1) / KX, (a.g.NY + KY - 1) / KY, coll ? a.g.NZ - 1 : a.g.NZ);
-    if (coll) k_turb_coll<T><<<grid, KX * KY, 0, s>>>(a);
-    else k_turb_stag<T><<<grid, KX * KY, 0, s>>>(a);
+    if (coll) launch_pdl(a.g.pdl, k_turb_coll<T>, grid, KX * KY, 0, s, a);
+    else launch_pdl(a.g.pdl, k_turb_stag<T>, grid, KX * KY, 0, s, a);
 }
 
 // ---------------------------------------------------------------------------
@@ -338,6 +346,8 @@ void launch_turb(const TurbArgs<T>& a, cudaStream_t s) {
 template <typename T, int SCHEME>
 __global__ void __launch_bounds__(256) k_divergence(DivArgs<T> a) {
     const Geom& g = a.g;
+    pdl_launch();
+    pdl_wait();
     const long long in = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (in >= g.N) return;
     const int ix = (int)(in % g.NX), iy = (int)((in / g.NX) % g.NY), iz = (int)(in / g.NXY);
@@ -347,9 +357,9 @@ __global__ void __launch_bounds__(256) k_divergence(DivArgs<T> a) {
 template <typename T>
 void launch_divergence(const DivArgs<T>& a, cudaStream_t s) {
     const unsigned nb = (unsigned)((a.g.N + 255) / 256);
-    if (a.g.scheme == TC_SCHEME_VV4) k_divergence<T, TC_SCHEME_VV4><<<nb, 256, 0, s>>>(a);
-    else if (a.g.scheme == TC_SCHEME_HW2) k_divergence<T, TC_SCHEME_HW2><<<nb, 256, 0, s>>>(a);
-    else k_divergence<T, TC_SCHEME_COLLOC><<<nb, 256, 0, s>>>(a);
+    if (a.g.scheme == TC_SCHEME_VV4) launch_pdl(a.g.pdl, k_divergence<T, TC_SCHEME_VV4>, nb, 256, 0, s, a);
+    else if (a.g.scheme == TC_SCHEME_HW2) launch_pdl(a.g.pdl, k_divergence<T, TC_SCHEME_HW2>, nb, 256, 0, s, a);
+    else launch_pdl(a.g.pdl, k_divergence<T, TC_SCHEME_COLLOC>, nb, 256, 0, s, a);
 }
 
 // ---------------------------------------------------------------------------
@@ -362,13 +372,18 @@ void launch_divergence(const DivArgs<T>& a, cudaStream_t s) {
 constexpr int NDIAG = NDIAG_SUMS;
 static_assert(NDIAG + 3 == TC_DIAG_STRIDE, "diagnostics layout");
 
-// Stage 1: CTA (z, s) reduces chunk s of plane z into part[(z*S + s)*STRIDE + k];
-// stage 2 sums the S chunks of every (z, k) in index order (deterministic).  Chunks
+// CTA (z, s) reduces chunk s of plane z into part[(z*S + s)*STRIDE + k].  The S chunks are
+// added in index order (deterministic) into planes, which may be pinned host memory: FIN, by
+// the plane's last CTA (small grids, where a second kernel and a copy back took 7 us of a
+// 64x64x64 step's 84); else by k_diag_finish (the fence and ticket of every CTA cost more on
+// large grids: 0.141 against 0.125 ms at 384x384x256 mixed).  Chunks
 // are multiples of 4 cells (NX*NY is), read as 16-byte vectors of 4 cells, so each
 // thread keeps 5-6 vector loads in flight per iteration.
-template <typename T>
+template <typename T, bool FIN>
 __global__ void __launch_bounds__(256) k_diag(DiagArgs<T> a, double* part, int S) {
     const Geom& g = a.g;
+    pdl_launch();
+    pdl_wait();
     const int z = blockIdx.x, s = blockIdx.y;
     const int NX = g.NX, NZ = g.NZ;
     const size_t NXY = (size_t)NX * g.NY;
@@ -447,7 +462,26 @@ __global__ void __launch_bounds__(256) k_diag(DiagArgs<T> a, double* part, int S
         const int k = threadIdx.x;
         double r = sb[k][0];
         for (int w2 = 1; w2 < (int)(blockDim.x >> 5); w2++) r = k < NDIAG ? r + sb[k][w2] : fmax(r, sb[k][w2]);
-        part[((size_t)z * S + s) * TC_DIAG_STRIDE + k] = r;
+        if (FIN && S == 1) a.planes[(size_t)z * TC_DIAG_STRIDE + k] = r;
+        else part[((size_t)z * S + s) * TC_DIAG_STRIDE + k] = r;
+    }
+    if constexpr (FIN) {
+        if (S == 1) return;
+        __shared__ bool last;
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) last = atomicAdd(a.ticket + z, 1u) == (unsigned)(S - 1);
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+        if (threadIdx.x < NDIAG + 3) {
+            const int k = threadIdx.x;
+            const volatile double* q = part + (size_t)z * S * TC_DIAG_STRIDE + k;
+            double r = q[0];
+            for (int c = 1; c < S; c++) r = k < NDIAG ? r + q[(size_t)c * TC_DIAG_STRIDE] : fmax(r, q[(size_t)c * TC_DIAG_STRIDE]);
+            a.planes[(size_t)z * TC_DIAG_STRIDE + k] = r;
+        }
+        if (threadIdx.x == 0) a.ticket[z] = 0u;  // for the next pass
     }
 }
 
@@ -686,9 +720,12 @@ void launch_diag_finish(const double* part, double* planes, int NZ, int S, cudaS
 template <typename T>
 void launch_diag(const DiagArgs<T>& a, cudaStream_t s) {
     const int S = diag_chunks(a.g);
-    k_diag<T><<<dim3(a.g.NZ, S), 256, 0, s>>>(a, a.part, S);
-    const int n = a.g.NZ * TC_DIAG_STRIDE;
-    k_diag_finish<<<(n + 255) / 256, 256, 0, s>>>(a.part, a.planes, a.g.NZ, S);
+    if (a.g.pdl) {
+        launch_pdl(true, k_diag<T, true>, dim3(a.g.NZ, S), 256, 0, s, a, a.part, S);
+        return;
+    }
+    k_diag<T, false><<<dim3(a.g.NZ, S), 256, 0, s>>>(a, a.part, S);
+    launch_diag_finish(a.part, a.planes, a.g.NZ, S, s);
 }
 
 // ---------------------------------------------------------------------------

@@ -290,7 +290,7 @@ static int mlp_grad_pass(const float* P, const float* X, const float* Y, long lo
     const int nb = mlp_grad_blocks(n);
     const size_t smem = sizeof(MlpTrainSmem);
     cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_pdl(k_mlp_grad, nb, MW * 32, smem, s, P, X, Y, n, part);
+    launch_pdl(true, k_mlp_grad, nb, MW * 32, smem, s, P, X, Y, n, part);
     return nb;
 }
 
@@ -305,7 +305,7 @@ void launch_mlp_step(float* P, float* M, float* V, const float* X, const float* 
     const int nb = mlp_grad_pass(P, X, Y, n, part, s);
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
-    launch_pdl(k_mlp_update, (MLP_NPAR + 1 + MLP_UNT - 1) / MLP_UNT, MLP_UNT, 0, s, part, nb, P, M, V, loss, lr, b1, b2, 1e-8f,
+    launch_pdl(true, k_mlp_update, (MLP_NPAR + 1 + MLP_UNT - 1) / MLP_UNT, MLP_UNT, 0, s, part, nb, P, M, V, loss, lr, b1, b2, 1e-8f,
                c1, c2);
 }
 

@@ -48,6 +48,8 @@ __global__ void __launch_bounds__(SRX* SRY, 2) k_srk_stage(SrkStage<T> a) {
     constexpr int MT = TC_SRK_MAX_STAGES;  // terms besides the first
     using V = Vw<T, W>;
     const Geom& g = a.g;
+    pdl_launch();
+    pdl_wait();
     const int NX = g.NX, NY = g.NY, NZ = g.NZ;
     const size_t NXY = (size_t)NX * NY, N = (size_t)g.N;
     const int x = W * (blockIdx.x * SRX + threadIdx.x % SRX), iy = blockIdx.y * SRY + threadIdx.x / SRX, z = blockIdx.z;
@@ -193,8 +195,8 @@ template <typename T, int W>
 static void srk_stage_w(const SrkStage<T>& a, cudaStream_t s) {
     const int nq = (a.g.NX + W - 1) / W;
     const dim3 grid((nq + SRX - 1) / SRX, (a.g.NY + SRY - 1) / SRY, a.g.NZ);
-    if (a.gb) k_srk_stage<T, W, true><<<grid, SRX * SRY, 0, s>>>(a);
-    else k_srk_stage<T, W, false><<<grid, SRX * SRY, 0, s>>>(a);
+    if (a.gb) launch_pdl(a.g.pdl, k_srk_stage<T, W, true>, grid, SRX * SRY, 0, s, a);
+    else launch_pdl(a.g.pdl, k_srk_stage<T, W, false>, grid, SRX * SRY, 0, s, a);
 }
 
 template <typename T>

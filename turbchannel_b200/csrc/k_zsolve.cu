@@ -515,6 +515,17 @@ __device__ __forceinline__ void zsolve_tile(const ZSolveArgs<T>& a, unsigned cha
     auto stored = [&](int i) {  // stored row of row i
         return i < top ? hr - top + i : (i < top + NB ? 2 * hr + i - top : 2 * hr - bot + (NZ - 1 - i));
     };
+    if constexpr (FS) {  // factors: one contiguous block, no kernel's output
+        constexpr int RB = KP * NV * (int)sizeof(C), W = RB % 16 == 0 ? 16 : 8;
+        const unsigned char* src = reinterpret_cast<const unsigned char*>(fac);
+        unsigned char* dst = reinterpret_cast<unsigned char*>(F);
+        const int n = rows * RB;
+#pragma unroll 4
+        for (int e = threadIdx.x * W; e < n; e += ZS_NT * W) cp_async<W>(dst + e, src + e);
+    }
+    for (int i = r0; i < 2 * hr - top - bot; i += RSTEP)  // rows of padding
+        xs[(i < hr - top ? i : hr + i - (hr - top)) * NM] = {C(0), C(0)};
+    pdl_wait();
     if (valid) {
         const cplx<T>* src = col + (size_t)r0 * M;
 #pragma unroll 4
@@ -526,16 +537,6 @@ __device__ __forceinline__ void zsolve_tile(const ZSolveArgs<T>& a, unsigned cha
                 xs[stored(i) * NM] = {(C)v.x, (C)v.y};
             }
         }
-    }
-    for (int i = r0; i < 2 * hr - top - bot; i += RSTEP)  // rows of padding
-        xs[(i < hr - top ? i : hr + i - (hr - top)) * NM] = {C(0), C(0)};
-    if constexpr (FS) {  // factors: one contiguous block
-        constexpr int RB = KP * NV * (int)sizeof(C), W = RB % 16 == 0 ? 16 : 8;
-        const unsigned char* src = reinterpret_cast<const unsigned char*>(fac);
-        unsigned char* dst = reinterpret_cast<unsigned char*>(F);
-        const int n = rows * RB;
-#pragma unroll 4
-        for (int e = threadIdx.x * W; e < n; e += ZS_NT * W) cp_async<W>(dst + e, src + e);
     }
     cp_async_commit();
     cp_async_wait<0>();
@@ -582,6 +583,7 @@ __global__ void __launch_bounds__(ZS_NT) k_zsolve_col(ZSolveArgs<T> a, int nlow,
     extern __shared__ __align__(32) unsigned char smz[];
     __shared__ __align__(16) double mid[2 * 3 * 32];
     const Geom& g = a.g;
+    pdl_launch();
     const int LM = g.low_modes, NZ = g.NZ, NYH1 = g.NY / 2 + 1;
     if constexpr (sizeof(T) == 4) {
         if ((int)blockIdx.x < nlow) {
@@ -615,8 +617,8 @@ static void zsolve_kp(const ZSolveArgs<T>& a, cudaStream_t s) {
         if (smem > ZS_SMEM_MAX) return zsolve_kp<T, VV, 1, false>(a, s);
     }
     auto k = k_zsolve_col<T, VV, KP, FS>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k<<<(unsigned)(nlow + (size_t)g.NXH * nkt), ZS_NT, smem, s>>>(a, nlow, nkl, nkt);
+    smem_limit(k, smem);
+    launch_pdl(a.g.pdl, k, (unsigned)(nlow + (size_t)g.NXH * nkt), ZS_NT, smem, s, a, nlow, nkl, nkt);
 }
 
 // ---------------------------------------------------------------------------
@@ -630,6 +632,8 @@ __global__ void __launch_bounds__(128) k_zsolve_stream(ZSolveArgs<double> a) {
     constexpr int R = 2;
     using C = cplx<double>;
     const Geom& g = a.g;
+    pdl_launch();
+    pdl_wait();
     const int NY = g.NY, NYH1 = NY / 2 + 1, NZ = g.NZ;
     const size_t M = (size_t)g.NXH * NY, MH = (size_t)g.NXH * NYH1;
     const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -922,7 +926,7 @@ int launch_zsolve_fac(const ZSolveArgs<T>& a, cudaStream_t s, cudaStream_t side,
     if constexpr (sizeof(T) == 8) {
         if (zs_stream(a.g, sizeof(T))) {
             const size_t n = (size_t)2 * a.g.NXH * (a.g.NY / 2 + 1);
-            k_zsolve_stream<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(a);
+            launch_pdl(a.g.pdl, k_zsolve_stream, (unsigned)((n + 127) / 128), 128, 0, s, a);
             return 1;
         }
     }

@@ -169,8 +169,9 @@ struct DiagArgs {
     const T* p;
     const T* nu_t;
     double tau;
-    double* planes;  // NZ x TC_DIAG_STRIDE
+    double* planes;  // NZ x TC_DIAG_STRIDE, device or pinned host memory
     double* part;    // NZ x diag_chunks() x TC_DIAG_STRIDE partial sums
+    unsigned* ticket;  // NZ zeros: CTAs of a plane that are done
 };
 constexpr int TC_DIAG_STRIDE = 19;
 constexpr int NDIAG_SUMS = 16;  // planes[z][0..15] are sums, [16..18] CFL maxima

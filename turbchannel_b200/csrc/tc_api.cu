@@ -219,6 +219,7 @@ struct tc_handle {
     RunCtl* run_ctl = nullptr;
     double run_tau = 0.0;
     int run_cur = -1, run_every = 0, run_mode = 0;
+    unsigned* diag_ticket = nullptr;  // per plane: chunks of the diagnostics pass that are done
     double* diag_part = nullptr;  // per-chunk partial sums of the diagnostics
     double* planes_h = nullptr;  // pinned
     double* stage = nullptr;     // AoS double staging (3N), lazily
@@ -317,7 +318,7 @@ static const cplx<T>* twy(const tc_handle* h) { return (const cplx<T>*)h->tw + h
 
 static void free_all(tc_handle* h) {
     void* ptrs[] = {h->nu_t, h->ptmp, h->spec, h->zfac, h->zfac_low, h->mesh_t, h->fk, h->stats, h->mesh_d, h->tabs, h->tw, h->red, h->ticket,
-                    h->err_flag, h->planes, h->diag_part, h->stage, h->opv, h->opf, h->ops, h->mlp_params, h->les_buf, h->fdiag_part,
+                    h->err_flag, h->planes, h->diag_part, h->diag_ticket, h->stage, h->opv, h->opf, h->ops, h->mlp_params, h->les_buf, h->fdiag_part,
                     h->srk.buf};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -503,6 +504,7 @@ extern "C" int tc_create(const tc_params* prm, const double* zz, tc_handle** out
     g.NX = p.NX; g.NY = p.NY; g.NZ = p.NZ; g.NXY = p.NX * p.NY;
     g.N = (long long)g.NXY * p.NZ;
     g.NXH = p.NX / 2 + 1;
+    g.pdl = g.N * (p.precision == TC_FP64 ? 8 : 4) <= TC_PDL_BYTES;
     g.scheme = p.scheme; g.visc_type = p.visc_type; g.turb = p.turb_model; g.stab_type = p.stab_type; g.fd_mode = p.fd_mode;
     int lm = p.low_modes > 0 ? p.low_modes : 4;
     lm = std::min(lm, std::min(g.NXH, (p.NY + 1) / 2));
@@ -638,6 +640,8 @@ extern "C" int tc_create(const tc_params* prm, const double* zz, tc_handle** out
     TC_ALLOC(h->planes, (size_t)g.NZ * TC_DIAG_STRIDE * sizeof(double));
     TC_ALLOC(h->stats, ((size_t)g.NZ * 12 + 1) * sizeof(double));
     cudaMemset(h->stats, 0, ((size_t)g.NZ * 12 + 1) * sizeof(double));
+    TC_ALLOC(h->diag_ticket, (size_t)g.NZ * sizeof(unsigned));
+    cudaMemset(h->diag_ticket, 0, (size_t)g.NZ * sizeof(unsigned));
     TC_ALLOC(h->diag_part, (size_t)g.NZ * diag_chunks(g) * TC_DIAG_STRIDE * sizeof(double));
     if (cudaMallocHost((void**)&h->planes_h, (size_t)g.NZ * TC_DIAG_STRIDE * sizeof(double)) != cudaSuccess) {
         free_all(h); delete h;
@@ -1123,12 +1127,11 @@ static int diag_run(tc_handle* h, int level, double tau) {
     a.p = (const T*)h->pres[level];
     a.nu_t = (h->nu_t && h->turb_kind != TC_TURB_NONE) ? (const T*)h->nu_t : nullptr;
     a.tau = tau;
-    a.planes = h->planes;
+    a.planes = h->planes_h;  // written by the kernel itself
     a.part = h->diag_part;
+    a.ticket = h->diag_ticket;
     launch_diag<T>(a, h->st);
     TC_CUDA(cudaGetLastError());
-    TC_CUDA(cudaMemcpyAsync(h->planes_h, h->planes, (size_t)h->g.NZ * TC_DIAG_STRIDE * sizeof(double),
-                            cudaMemcpyDeviceToHost, h->st));
     TC_CUDA(cudaStreamSynchronize(h->st));
     return TC_OK;
 }
@@ -1149,6 +1152,7 @@ static int diag_device(tc_handle* h, int level) {
         a.tau = 0.0;
         a.planes = h->planes;
         a.part = h->diag_part;
+        a.ticket = h->diag_ticket;
         launch_diag<T>(a, h->st);
     }
     TC_CUDA(cudaGetLastError());
@@ -2200,6 +2204,7 @@ static int run_capture_body(tc_handle* h, double tau, int cur, int every, int mo
     a.tau = tau;
     a.planes = h->planes;
     a.part = h->diag_part;
+    a.ticket = h->diag_ticket;
     launch_diag<T>(a, h->st);
     launch_run_ctl(hnd, h->planes, h->g.NZ, mode, h->run_ctl, h->st);
     return check_launch("tc_run_graph");

@@ -11,6 +11,7 @@ namespace tc {
 // ---------------------------------------------------------------------------
 // Plain data passed to kernels by value
 // ---------------------------------------------------------------------------
+constexpr long long TC_PDL_BYTES = 48ll << 20;
 struct Geom {
     int NX, NY, NZ, NXY;
     long long N;  // cells (or nodes)
@@ -21,6 +22,13 @@ struct Geom {
     // (collocated_AB3/func_global.h:163-170), 1 shift sum(p vol) / area
     // (collocated_SRK/func_global.h:130-137)
     int norm_srk = 0;
+    // programmatic launches between the step's kernels: fields up to TC_PDL_BYTES.  There the
+    // gaps between kernels are a large part of the step (64x64x64 FP64 with diagnostics 83.5 ->
+    // 73.5 us, 216x108x95 mixed 185 -> 168, 128x64x49 SRK 283 -> 230; up to 192x192x128 and
+    // 256x192x128 FP64, 36 and 48 MB a field, 385 -> 373 and 489 -> 485).  On larger grids CTAs
+    // of the next kernel take room from the running one: 256x256x192 FP64 931 -> 955 us,
+    // 384x384x256 mixed 1.61 -> 1.67 ms, FP64 3.60 -> 4.05 ms.
+    bool pdl = false;
 };
 
 // Mesh-derived arrays (device pointers into one allocation).  Staggered arrays
@@ -105,7 +113,7 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
 template <typename... P, typename... A>
-static inline void launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+static inline void launch_pdl(bool on, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
     cudaLaunchConfig_t c = {};
     c.gridDim = grid;
     c.blockDim = block;
@@ -115,8 +123,14 @@ static inline void launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t 
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     c.attrs = at;
-    c.numAttrs = 1;
+    c.numAttrs = on ? 1 : 0;  // off: an ordinary launch, whose pdl_wait returns at once
     cudaLaunchKernelEx(&c, kern, P(args)...);
+}
+
+// Dynamic shared memory beyond the 48 KB every kernel may use has to be allowed.
+template <typename K>
+static inline void smem_limit(K kern, size_t bytes) {
+    if (bytes > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 // ---------------------------------------------------------------------------

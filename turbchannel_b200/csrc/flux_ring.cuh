@@ -4,9 +4,28 @@
 // the periodic wrap moves whole 16-byte chunks) sit in a ring of 2H+2 slots, and the next
 // plane is fetched with LDGSTS (cp.async) while the current one is computed.
 #pragma once
+#include <algorithm>
+
 #include "tc_common.cuh"
 
 namespace tc {
+
+// Planes per CTA of a kernel with `tiles` tiles per plane and `ctas` CTAs per SM: one
+// wave of CTAs where the tiles leave room for it -- every further one refills its ring and
+// ends in a partly empty wave (8 chunks per SM before: VV4 FP64 192x192x96 216 -> 188 us,
+// 96x96x96 67 -> 56, 192x192x256 527 -> 477; HW2 LES 192x192x128 mixed 122 -> 111; collocated
+// 128x128x128 mixed 48 -> 40) -- or two waves of tall chunks where one would leave some SMs
+// with a single CTA (collocated 256x256x192 FP64, 256 tiles: one chunk 353 us, two 333,
+// eight per SM 344; at 96 and 128 planes one chunk is the faster); more tiles than that: 8
+// chunks per SM (384x384x256 FP64, 576 tiles).
+static inline int flux_chunk(int tiles, int NZ, int ctas = 2) {
+    const int slots = 148 * ctas;
+    int nch;
+    if (tiles > slots) nch = (148 * 8 + tiles - 1) / tiles;
+    else if (2 * tiles > slots && NZ >= 160) nch = 2 * slots / tiles;
+    else nch = slots / tiles;
+    return std::max(4, (NZ + nch - 1) / nch);
+}
 
 constexpr int STX = 32, STY = 8;  // threads per CTA: 32 x 8
 constexpr int SG = 4;              // x-halo of the shared tile (a whole 16-byte chunk for float and double)

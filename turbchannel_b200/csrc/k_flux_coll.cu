@@ -84,8 +84,14 @@ __device__ __forceinline__ void visc_galerkin(const ACC& A, const NUT& nut, int 
 }
 
 // CY: nodes per thread along y (the tile is 32 x 8 CY nodes): two for float, one for double.
+// CTAs per SM: the float operator form (the SRK step's explicit term), which holds no history
+// and was bound by its instructions at 62% of the issue rate with two, takes three
+// (384x384x257: 326 -> 306 us).
+template <typename T, int VISC, int ORDER>
+constexpr int coll_ctas() { return sizeof(T) == 4 && VISC == TC_VISC_CROSS && ORDER == 0 ? 3 : 2; }
+
 template <typename T, int VISC, bool LES, int ORDER, bool STAB1, bool VEC, int CY>
-__global__ void __launch_bounds__(STX* STY, 2) k_flux_coll(FluxArgs<T> a, int tz) {
+__global__ void __launch_bounds__(STX* STY, coll_ctas<T, VISC, ORDER>()) k_flux_coll(FluxArgs<T> a, int tz) {
     pdl_launch();
     pdl_wait();
     using ACC = RingAcc<T, 1, CY>;
@@ -250,11 +256,10 @@ __global__ void __launch_bounds__(STX* STY, 2) k_flux_coll(FluxArgs<T> a, int tz
 template <typename T>
 constexpr int coll_cy() { return sizeof(T) == 4 ? 2 : 1; }
 
-static void flux_coll_shape(const Geom& g, int cy, dim3& grid, int& tz) {
+static void flux_coll_shape(const Geom& g, int cy, int ctas, dim3& grid, int& tz) {
     const int ty = STY * cy;
     const int tiles = ((g.NX + STX - 1) / STX) * ((g.NY + ty - 1) / ty);
-    int nch = std::max(1, (148 * 8 + tiles - 1) / tiles);
-    tz = std::max(4, (g.NZ + nch - 1) / nch);
+    tz = flux_chunk(tiles, g.NZ, ctas);
     grid = dim3((g.NX + STX - 1) / STX, (g.NY + ty - 1) / ty, (g.NZ + tz - 1) / tz);
 }
 
@@ -267,7 +272,7 @@ static void run(const FluxArgs<T>& a, cudaStream_t s) {
     smem_limit(kern, smem);
     dim3 grid;
     int tz;
-    flux_coll_shape(a.g, CY, grid, tz);
+    flux_coll_shape(a.g, CY, coll_ctas<T, VISC, ORDER>(), grid, tz);
     launch_pdl(a.g.pdl, kern, grid, STX * STY, smem, s, a, tz);
 }
 

@@ -184,18 +184,13 @@ constexpr int flux_ty() { return STY; }
 static void flux_stag_shape(const Geom& g, int tile_rows, dim3& grid, int& tz) {
     const int ty = tile_rows;
     const int tiles = ((g.NX + STX - 1) / STX) * ((g.NY + ty - 1) / ty);
-    int nch = std::max(1, (148 * 8 + tiles - 1) / tiles);
-    tz = std::max(4, (g.NZ + nch - 1) / nch);
+    tz = flux_chunk(tiles, g.NZ);
     grid = dim3((g.NX + STX - 1) / STX, (g.NY + ty - 1) / ty, (g.NZ + tz - 1) / tz);
 }
 
-// upper bound of the flux kernels' grid sizes (sizes the partial-sum buffer)
-int flux_grid_blocks(const Geom& g) {
-    dim3 gr;
-    int tz;
-    flux_stag_shape(g, STY, gr, tz);  // the smallest tile of the kernels
-    return (int)(gr.x * gr.y * gr.z);
-}
+// upper bound of the flux kernels' grid sizes (sizes the partial-sum buffer): every kernel has
+// at most max(592, 1184 + tiles) CTAs (flux_chunk), the smallest tile being 32 x 8
+int flux_grid_blocks(const Geom& g) { return 2 * 1184 + ((g.NX + STX - 1) / STX) * ((g.NY + STY - 1) / STY); }
 
 template <typename T, int SCHEME, int VISC, bool LES, int ORDER>
 static void run(const FluxArgs<T>& a, cudaStream_t s) {

@@ -4,10 +4,10 @@
 // right-hand side K_i - G buf + alpha v - d_i nu1 (one pass of this kernel), the pressure
 // solve, and one pass that forms p_i = mu + buf, mu_i, q_i, K_i - G p_i, the next stage's
 // velocity and the next stage's buf and p-hat.
-// Bound by DRAM: the passes of a four-stage ARS step move about 120 words per node (3.7 ms at
-// 384x384x257 mixed, 75% of the copy bandwidth).  As separate gradient, linear-combination
+// Bound by DRAM: the passes of a four-stage ARS step move about 120 words per node (3.1 ms at
+// 384x384x257 mixed, 90% of the copy bandwidth).  As separate gradient, linear-combination
 // and scalar kernels they moved 173 (4.4 ms) and took 17 launches more; the step with its
-// diagnostics went from 7.28 to 6.50 ms, at 128x64x49 FP64 from 0.354 to 0.29 ms.
+// diagnostics went from 7.28 to 5.84 ms, at 128x64x49 FP64 from 0.354 to 0.21 ms.
 #include <algorithm>
 
 #include "kernels.cuh"
@@ -43,8 +43,11 @@ constexpr int SRX = 32, SRY = 8;  // threads along x (W nodes each) and rows per
 // SUM: the gradient's field is ga + gb (rounded), else ga.  Every load of a part is issued
 // before its arithmetic: with one load per trip of a run-time loop the pass waited for
 // memory (384x384x257 mixed: 0.98 / 0.49 ms per pass with / without SUM against 0.80 / 0.32).
+// CTAs per SM: what still waits is hidden by more warps.  Three in place of two take 80
+// registers a thread: 0.67 / 0.27 ms mixed, and FP64 256x192x128 1.86 to 1.67 ms per step;
+// four, at 64, give the pass without SUM another 6% and spill 26 words of the one with it.
 template <typename T, int W, bool SUM>
-__global__ void __launch_bounds__(SRX* SRY, 2) k_srk_stage(SrkStage<T> a) {
+__global__ void __launch_bounds__(SRX* SRY, sizeof(T) == 4 && !SUM ? 4 : 3) k_srk_stage(SrkStage<T> a) {
     constexpr int MT = TC_SRK_MAX_STAGES;  // terms besides the first
     using V = Vw<T, W>;
     const Geom& g = a.g;

@@ -47,3 +47,22 @@ def test_pressure_solve_length(NX, NY, precision):
     S.close()
     err = np.linalg.norm(got - want) / np.linalg.norm(want)
     assert within(f"fft/{NX}x{NY}/p1", err, 2.4e-6), err
+
+
+@pytest.mark.parametrize("NX", [384, 512, 768, 972, 1024])
+def test_inverse_x_tiles(NX):
+    """The float inverse x-transform with several tiles per CTA: the first pass over its own
+    tile (two CTAs per SM at 512, one at 1024), in a buffer of its own (768), and with more
+    line segments than threads (972).  The bound is the one above."""
+    import oracle_py as op
+    import turbchannel_b200 as tb
+
+    prod, orc, zz = make_case(HW2, NX, 1024, 7, precision=1)
+    S = tb.Solver(prod, zz)
+    r32 = np.random.default_rng(23).standard_normal(S.N)
+    r32 = (r32 - r32.mean()).astype(np.float32).astype(np.float64)
+    want = op.Oracle(orc, zz, "f64").pressure_solve(r32)
+    got = S.LinearSystemSolveFFT(r32)
+    S.close()
+    err = np.linalg.norm(got - want) / np.linalg.norm(want)
+    assert within(f"fft/{NX}x1024/p1/tiles", err, 2.4e-6), err

@@ -162,17 +162,47 @@ static void xfft_reg_launch(const DivFftArgs<T>& a, const T* src, int rows, cuda
 // inverse x-FFT, persistent and double-buffered (float)
 // ---------------------------------------------------------------------------
 constexpr int XP_NT = 256;
-// As k_ixfft_reg (the Hermitian-extended
-// half spectrum of two rows per complex line, inverse transform, scaled rows into p), with
-// each CTA walking tiles of RB (16) y-values of one plane and copying the next tile's half
-// spectrum (NX/2+1 rows of RB contiguous values) into its second buffer while it
-// transforms the current one.
+// Shared memory of an SM's CTAs, at most: the rest is the L1 that the twiddle factors stay in
+// (512x512x256 float: 145 us with two CTAs of 107 KB, 114 with two of 74 KB).
+constexpr size_t XP_SMEM = 204 * 1024;
+// Row stride of a tile of half spectra, tile[kx * stride + row]: neighbouring lanes gather
+// the 16 bytes of two rows (float; one row in double) of neighbouring kx, which this stride
+// spreads over all banks.
+template <typename T>
+__host__ __device__ constexpr int ixfft_stride(int rows) {
+    return sizeof(T) == 4 ? (rows / 2 | 1) * 2 : rows | 1;
+}
+// rows r, r + 1 of a tile row (r even)
+template <typename T>
+__device__ __forceinline__ void ld_rows(const cplx<T>* t, cplx<T>& a, cplx<T>& b) {
+    if constexpr (sizeof(T) == 4) {
+        const float4 q = *reinterpret_cast<const float4*>(t);
+        a = {q.x, q.y};
+        b = {q.z, q.w};
+    } else {
+        a = t[0];
+        b = t[1];
+    }
+}
+
+// As k_ixfft_reg (the Hermitian-extended half spectrum of two rows per complex line, inverse
+// transform, scaled rows into p), with each CTA walking tiles of RB (16) y-values of one plane
+// and copying the next tile's half spectrum (NX/2+1 rows of RB contiguous values) into its
+// second buffer while it transforms the current one.  Bound by DRAM, 4.8 TB/s at 512x512x256
+// float (0.114 ms) and 4.5 at 384x384x256 (0.068).
 template <typename T, int N>
 struct IPipe {
-    static constexpr int RB = sizeof(T) == 4 ? 16 : 8, NL = RB / 2, TS = RB + 2, NXH = N / 2 + 1;
+    static constexpr int RB = sizeof(T) == 4 ? 16 : 8, NL = RB / 2, TS = ixfft_stride<T>(RB), NXH = N / 2 + 1;
     static constexpr int PC = 16 / sizeof(cplx<T>), CPK = RB / PC;  // 16-byte chunks per kx row
-    static constexpr size_t buf = ((size_t)NXH * TS * sizeof(cplx<T>) + 15) / 16 * 16;
-    static constexpr size_t smem = 2 * buf + (size_t)NL * FftSplit<N>::YL * sizeof(cplx<T>);
+    static constexpr size_t tile = (size_t)NXH * TS * sizeof(cplx<T>), y = (size_t)NL * FftSplit<N>::YL * sizeof(cplx<T>);
+    static constexpr size_t shared = 2 * (tile > y ? tile : y), own = 2 * tile + y;
+    // alias: the first pass is written over the tile it was gathered from (every thread holds
+    // at most one line segment), else to a buffer of its own after the two tiles.  It costs a
+    // barrier, and is worth it for the shared memory: not where that still gives one CTA per
+    // SM either way (NX = 768: 82 us with a buffer, 104 without at 768x384x128).
+    static constexpr bool alias = NL * FftSplit<N>::N2 <= XP_NT && (2 * shared <= XP_SMEM || own > XP_SMEM);
+    static constexpr size_t buf = ((alias ? shared / 2 : tile) + 15) / 16 * 16;
+    static constexpr size_t smem = 2 * buf + (alias ? 0 : y);
 };
 
 template <typename T, int N>
@@ -181,7 +211,6 @@ __global__ void __launch_bounds__(XP_NT) k_ixfft_pipe(IxFftArgs<T> a) {
     constexpr int RB = P::RB, NL = P::NL, TS = P::TS, NXH = P::NXH, PC = P::PC, CPK = P::CPK;
     constexpr int N1 = FftSplit<N>::N1, N2 = FftSplit<N>::N2, YL = FftSplit<N>::YL, NH = N / 2;
     extern __shared__ __align__(16) unsigned char smraw[];
-    cplx<T>* Y = reinterpret_cast<cplx<T>*>(smraw + 2 * P::buf);
     const Geom& g = a.g;
     const int NY = g.NY, YB = NY / RB;
     const long long ntile = (long long)YB * g.NZ;
@@ -209,16 +238,16 @@ __global__ void __launch_bounds__(XP_NT) k_ixfft_pipe(IxFftArgs<T> a) {
         cp_async_wait<1>();
         __syncthreads();  // tile t is in buffer b
         const int z = (int)(t / YB), y0 = (int)(t - (long long)z * YB) * RB;
-        const cplx<T>* tile = reinterpret_cast<const cplx<T>*>(smraw + b * P::buf);
-        for (int it = threadIdx.x; it < NL * N2; it += XP_NT) {
-            const int l = it / N2, n2 = it - l * N2;
-            cplx<T> v[N1];
+        cplx<T>* tile = reinterpret_cast<cplx<T>*>(smraw + b * P::buf);
+        cplx<T>* Y = P::alias ? tile : reinterpret_cast<cplx<T>*>(smraw + 2 * P::buf);
+        // the Hermitian-extended line of rows 2l, 2l+1 at the first pass's positions
+        auto gather = [&](int l, int n2, cplx<T>(&v)[N1]) {
 #pragma unroll
-            for (int n1 = 0; n1 < N1; n1++) {  // the Hermitian-extended line of rows 2l, 2l+1
+            for (int n1 = 0; n1 < N1; n1++) {
                 const int k = N2 * n1 + n2;
                 const bool up = k > NH;
-                const cplx<T>* tp = tile + (up ? N - k : k) * TS + 2 * l;
-                cplx<T> av = tp[0], bv = tp[1];
+                cplx<T> av, bv;
+                ld_rows(tile + (up ? N - k : k) * TS + 2 * l, av, bv);
                 if (up) {
                     av.y = -av.y;
                     bv.y = -bv.y;
@@ -229,7 +258,21 @@ __global__ void __launch_bounds__(XP_NT) k_ixfft_pipe(IxFftArgs<T> a) {
                 }
                 v[n1] = {av.x - bv.y, av.y + bv.x};
             }
-            fft_pass_a<T, N, +1>(v, n2, a.twx, Y + l * YL);
+        };
+        if constexpr (P::alias) {
+            const bool mine = (int)threadIdx.x < NL * N2;
+            const int l = threadIdx.x / N2, n2 = threadIdx.x - l * N2;
+            cplx<T> v[N1];
+            if (mine) gather(l, n2, v);
+            __syncthreads();
+            if (mine) fft_pass_a<T, N, +1>(v, n2, a.twx, Y + l * YL);
+        } else {
+            for (int it = threadIdx.x; it < NL * N2; it += XP_NT) {
+                const int l = it / N2, n2 = it - l * N2;
+                cplx<T> v[N1];
+                gather(l, n2, v);
+                fft_pass_a<T, N, +1>(v, n2, a.twx, Y + l * YL);
+            }
         }
         __syncthreads();
         for (int it = threadIdx.x; it < NL * N1; it += XP_NT) {
@@ -244,7 +287,7 @@ __global__ void __launch_bounds__(XP_NT) k_ixfft_pipe(IxFftArgs<T> a) {
                 pb[k2 * N1] = v[k2].y * sc;
             }
         }
-        __syncthreads();  // buffer b and Y are refilled by the next iterations
+        __syncthreads();  // buffer b (and Y) are refilled by the next iterations
     }
 }
 
@@ -270,6 +313,7 @@ static bool ixfft_pipe_launch(const IxFftArgs<T>& a, cudaStream_t s) {
             if (P::smem <= (size_t)optin) {
                 cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::smem);
                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k, XP_NT, P::smem);
+                o = std::min(o, std::max(1, (int)(XP_SMEM / P::smem)));
             }
             sms_of[dev] = n;
             occ_of[dev] = o > 0 ? o : -1;
@@ -294,7 +338,7 @@ __global__ void __launch_bounds__(512) k_ixfft_reg(IxFftArgs<T> a, int rows, uns
     const Geom& g = a.g;
     pdl_launch();
     pdl_wait();
-    const int NY = g.NY, nl = rows >> 1, TS = rows + 2;
+    const int NY = g.NY, nl = rows >> 1, TS = ixfft_stride<T>(rows);
     cplx<T>* tile = reinterpret_cast<cplx<T>*>(smraw);  // tile[kx * TS + r]
     // alias: the first pass's output over the tile itself, every thread holding at most
     // one line segment (gather all, barrier, transform and write); else after the tile
@@ -318,7 +362,8 @@ __global__ void __launch_bounds__(512) k_ixfft_reg(IxFftArgs<T> a, int rows, uns
             const int k = N2 * n1 + n2;
             const bool up = k > NH;
             const cplx<T>* t = tile + (up ? N - k : k) * TS + 2 * l;
-            cplx<T> av = t[0], bv = t[1];
+            cplx<T> av, bv;
+            ld_rows(t, av, bv);
             if (up) {
                 av.y = -av.y;
                 bv.y = -bv.y;
@@ -377,7 +422,7 @@ static int ixfft_threads(int rows) {
 
 template <typename T, int N>
 static size_t ixfft_reg_smem(int rows) {
-    const size_t tile = (size_t)(N / 2 + 1) * (rows + 2), y = (size_t)(rows / 2) * FftSplit<N>::YL;
+    const size_t tile = (size_t)(N / 2 + 1) * ixfft_stride<T>(rows), y = (size_t)(rows / 2) * FftSplit<N>::YL;
     return (ixfft_alias<T, N>(rows) ? std::max(tile, y) : tile + y) * sizeof(cplx<T>);
 }
 

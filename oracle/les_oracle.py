@@ -12,7 +12,7 @@ checker of the CUDA kernels:
                     roundings (weights, inputs, hidden activations, backward factors)
 * smagorinsky_nut   the reference's algebraic model in the same wall units, as the
                     baseline the learned closure is compared with
-* adam_step         the optimiser of k_mlp_adam
+* adam_step         the optimiser of k_mlp_update
 
 Staggered layout: u on the lower x-face, v on the lower y-face, w on the lower z-face
 of a cell (w = 0 on both walls); cell-centred values are the two-face means.

@@ -5,8 +5,8 @@
 // spectrum buffer and the mesh-derived arrays, here on one CUDA device and one
 // stream.  Fields are stored structure-of-arrays in the working precision; the
 // boundary converts from/to the reference's AoS double layout.  One step is
-// seven launches (eight with a Smagorinsky model):
-//   flux+combine -> div+xFFT -> yFFT -> zsolve -> inverse yFFT -> inverse xFFT -> correction
+// eight launches (nine with a turbulence model):
+//   flux+combine -> divergence -> xFFT -> yFFT -> zsolve -> inverse yFFT -> inverse xFFT -> correction
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -127,10 +127,11 @@ static inline void launch_pdl(bool on, void (*kern)(P...), dim3 grid, dim3 block
     cudaLaunchKernelEx(&c, kern, P(args)...);
 }
 
-// Dynamic shared memory beyond the 48 KB every kernel may use has to be allowed.
+// A kernel's static and dynamic shared memory together may take 48 KB without asking.  The
+// question is put from 32 KB of dynamic memory on (no kernel here has 16 KB of static memory).
 template <typename K>
 static inline void smem_limit(K kern, size_t bytes) {
-    if (bytes > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (bytes > 32 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 // ---------------------------------------------------------------------------

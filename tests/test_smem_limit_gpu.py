@@ -70,3 +70,10 @@ def test_first_solver_of_a_process(tmp_path, scheme, NX, NY, NZ, precision):
         err = np.linalg.norm(_solve_in_child(tmp_path, scheme, NX, NY, NZ, precision, rhs) - want) / np.linalg.norm(want)
         tol = 2.4e-6 + 8 * 6e-8 * (NZ / 8) ** 1.5
     assert within(f"smem/{scheme}/{NX}x{NY}x{NZ}/p{precision}", err, tol), err
+
+
+def test_refused_launch_is_reported(tmp_path):
+    """A column that no tile holds: the z-solve's launch is refused, and the call says so although
+    it is the process's first and other kernels are set up after it."""
+    with pytest.raises(AssertionError, match="pressure_solve"):
+        _solve_in_child(tmp_path, VV4, 16, 16, 8000, 1, np.zeros(16 * 16 * 8000))

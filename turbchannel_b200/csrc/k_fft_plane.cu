@@ -302,7 +302,7 @@ static void plane_fwd(const T* src, cplx<T>* spec, const cplx<T>* twx, const cpl
     if constexpr (P::ok) {
         cudaLaunchAttribute at[2];
         const cudaLaunchConfig_t cfg = plane_config(at, pdl, nz, P::smem, s);
-        cudaLaunchKernelEx(&cfg, k_xyfft_plane<T, NX, NY>, src, spec, twx, twy);
+        note_launch(cudaLaunchKernelEx(&cfg, k_xyfft_plane<T, NX, NY>, src, spec, twx, twy));
     }
 }
 
@@ -313,7 +313,7 @@ static void plane_inv(const cplx<T>* spec, T* p, const cplx<T>* twx, const cplx<
     if constexpr (P::ok) {
         cudaLaunchAttribute at[2];
         const cudaLaunchConfig_t cfg = plane_config(at, pdl, nz, P::smem, s);
-        cudaLaunchKernelEx(&cfg, k_ixyfft_plane<T, NX, NY>, spec, p, twx, twy, scale);
+        note_launch(cudaLaunchKernelEx(&cfg, k_ixyfft_plane<T, NX, NY>, spec, p, twx, twy, scale));
     }
 }
 

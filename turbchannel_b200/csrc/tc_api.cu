@@ -690,6 +690,8 @@ extern "C" int tc_destroy(tc_handle* h) {
 
 static int check_launch(const char* what) {
     cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = launch_error;
+    launch_error = cudaSuccess;
     if (e != cudaSuccess) return fail(TC_E_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
     return TC_OK;
 }
@@ -1113,7 +1115,7 @@ static int diag_run(tc_handle* h, int level, double tau) {
     if (h->fused_valid && level == h->fused_level && tau == h->fused_tau) {
         launch_diag_finish(h->fdiag_part, h->planes, h->g.NZ, correct_diag_chunks(h->g), h->st);
         h->fused_used = true;
-        TC_CUDA(cudaGetLastError());
+        if (const int rc = check_launch("diagnostics")) return rc;
         TC_CUDA(cudaMemcpyAsync(h->planes_h, h->planes, (size_t)h->g.NZ * TC_DIAG_STRIDE * sizeof(double),
                                 cudaMemcpyDeviceToHost, h->st));
         TC_CUDA(cudaStreamSynchronize(h->st));
@@ -1131,7 +1133,7 @@ static int diag_run(tc_handle* h, int level, double tau) {
     a.part = h->diag_part;
     a.ticket = h->diag_ticket;
     launch_diag<T>(a, h->st);
-    TC_CUDA(cudaGetLastError());
+    if (const int rc = check_launch("diagnostics")) return rc;
     TC_CUDA(cudaStreamSynchronize(h->st));
     return TC_OK;
 }
@@ -1155,7 +1157,7 @@ static int diag_device(tc_handle* h, int level) {
         a.ticket = h->diag_ticket;
         launch_diag<T>(a, h->st);
     }
-    TC_CUDA(cudaGetLastError());
+    if (const int rc = check_launch("diagnostics")) return rc;
     return TC_OK;
 }
 
@@ -2157,8 +2159,7 @@ extern "C" int tc_stats_accumulate(tc_handle* h, int level, double weight) {
     int rc = TC_DISPATCH(h, diag_device, h, level);
     if (rc) return rc;
     launch_stats_acc(h->planes, h->stats, h->g.NZ, 1.0 / (double)h->g.NXY, weight, h->st);
-    TC_CUDA(cudaGetLastError());
-    return TC_OK;
+    return check_launch("tc_stats_accumulate");
 }
 
 extern "C" int tc_stats_read(tc_handle* h, double* profiles, double* total_weight) {

@@ -112,6 +112,14 @@ __host__ __device__ __forceinline__ cplx<T> cmul(cplx<T> a, cplx<T> b) {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
+// The first launch refused since the last check_launch (tc_api.cu).  The runtime's own last
+// error can be gone by then: a VV4 mixed 16x16x750 solve whose z-solve was refused returned
+// success, with the queries of the inverse x-FFT's first launch between the two.
+inline thread_local cudaError_t launch_error = cudaSuccess;
+static inline void note_launch(cudaError_t e) {
+    if (launch_error == cudaSuccess) launch_error = e;
+}
+
 template <typename... P, typename... A>
 static inline void launch_pdl(bool on, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
     cudaLaunchConfig_t c = {};
@@ -124,7 +132,7 @@ static inline void launch_pdl(bool on, void (*kern)(P...), dim3 grid, dim3 block
     at[0].val.programmaticStreamSerializationAllowed = 1;
     c.attrs = at;
     c.numAttrs = on ? 1 : 0;  // off: an ordinary launch, whose pdl_wait returns at once
-    cudaLaunchKernelEx(&c, kern, P(args)...);
+    note_launch(cudaLaunchKernelEx(&c, kern, P(args)...));
 }
 
 // A kernel's static and dynamic shared memory together may take 48 KB without asking.  The

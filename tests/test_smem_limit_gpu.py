@@ -77,3 +77,37 @@ def test_refused_launch_is_reported(tmp_path):
     it is the process's first and other kernels are set up after it."""
     with pytest.raises(AssertionError, match="pressure_solve"):
         _solve_in_child(tmp_path, VV4, 16, 16, 8000, 1, np.zeros(16 * 16 * 8000))
+
+
+def test_solvers_of_two_threads():
+    """Two threads, each with its own solver, both of them using the same tile kernel with columns
+    of different length: neither takes back the shared memory that the other has asked for."""
+    import threading
+
+    import torch
+
+    import turbchannel_b200 as tb
+
+    failed = []
+
+    def work(NZ):
+        try:
+            prod, _, zz = make_case(HW2, 16, 16, NZ, gamma=1.0)
+            S = tb.Solver(prod, zz)
+            r = torch.zeros(256 * NZ, device="cuda", dtype=torch.float64)
+            p = torch.empty_like(r)
+            torch.cuda.synchronize()
+            for k in range(3000):
+                S.pressure_solve_device(r.data_ptr(), p.data_ptr())
+                if k % 100 == 99:
+                    S.sync()
+            S.close()
+        except Exception as e:  # noqa: BLE001
+            failed.append((NZ, str(e)))
+
+    ts = [threading.Thread(target=work, args=(nz,)) for nz in (600, 1000)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not failed, failed

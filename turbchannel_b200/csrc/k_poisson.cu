@@ -69,7 +69,7 @@ int launch_div_xfft(const DivFftArgs<T>& a, cudaStream_t s) {
 #define TC_LDX(SCH, SC)                                                                                 \
     {                                                                                                   \
         auto k = rows == 8 ? k_div_xfft<T, SCH, SC, 8> : rows == 4 ? k_div_xfft<T, SCH, SC, 4> : k_div_xfft<T, SCH, SC, 2>; \
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);               \
+        smem_limit(k, smem);                                                                           \
         k<<<grid, 256, smem, s>>>(a);                                                                   \
     }
     if (a.src_scalar) TC_LDX(TC_SCHEME_HW2, true)
@@ -113,7 +113,7 @@ void launch_yfft(const YFftArgs<T>& a, cudaStream_t s) {
     const size_t smem = (size_t)2 * lines * a.g.NY * sizeof(cplx<T>);
     const long long total = (long long)a.g.NZ * a.g.NXH;
     auto k = k_yfft<T>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    smem_limit(k, smem);
     k<<<(unsigned)((total + lines - 1) / lines), 256, smem, s>>>(a, lines);
 }
 
@@ -459,7 +459,7 @@ static void zsolve_scheme(const ZSolveArgs<T>& a, cudaStream_t s, cudaStream_t s
         const int nma = SCHEME == TC_SCHEME_VV4 ? 3 * a.g.NZ : a.g.NZ;
         const size_t smem = (size_t)a.g.NZ * (sizeof(cplx<double>) + nc * sizeof(double)) + (size_t)(nma + 2 * a.g.NZ) * sizeof(double);
         auto k = k_zsolve_low<T, SCHEME>;
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        smem_limit(k, smem);
         k<<<nlow, 128, smem, side>>>(a);
         cudaEventRecord(join, side);
         k_zsolve_all<float, T, SCHEME><<<(unsigned)((M + 63) / 64), 64, 0, s>>>(a, 1);
@@ -529,7 +529,7 @@ void launch_ixfft(const IxFftArgs<T>& a, cudaStream_t s) {
     const size_t nl = rows / 2;
     const size_t smem = (nl * a.g.NX + std::max(nl * a.g.NX, (size_t)rows * a.g.NXH)) * sizeof(cplx<T>);
     auto k = rows == 8 ? k_ixfft<T, 8> : rows == 4 ? k_ixfft<T, 4> : k_ixfft<T, 2>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    smem_limit(k, smem);
     k<<<dim3(a.g.NY / rows, a.g.NZ), 256, smem, s>>>(a);
 }
 

@@ -68,7 +68,7 @@ static size_t zs_smem(const Geom& g, int kp, int eb, bool staged = true) {
 }
 static int zs_ktiles(const Geom& g, int kp) { return (g.NY / 2 + kp) / kp; }  // tiles of the NY/2+1 pairs of one kx
 constexpr size_t ZS_SMEM = 110 * 1024;  // at most, while a tile has two pairs or more: two CTAs per SM
-constexpr size_t ZS_SMEM_MAX = 223 * 1024;  // beyond (NZ of several thousand): factors stay in global memory
+constexpr size_t ZS_SMEM_MAX = SMEM_MOST;  // beyond (NZ of several thousand): factors stay in global memory
 constexpr int ZS_CTAS = 148 * 2;
 
 // Pairs per tile: 8 (64-byte rows in float), fewer where the columns are long (shared
@@ -617,7 +617,7 @@ static void zsolve_kp(const ZSolveArgs<T>& a, cudaStream_t s) {
         if (smem > ZS_SMEM_MAX) return zsolve_kp<T, VV, 1, false>(a, s);
     }
     auto k = k_zsolve_col<T, VV, KP, FS>;
-    smem_limit(k, smem);
+    smem_limit(k, smem, FS ? SMEM_MOST : SMEM_MOST + 2048);
     launch_pdl(a.g.pdl, k, (unsigned)(nlow + (size_t)g.NXH * nkt), ZS_NT, smem, s, a, nlow, nkl, nkt);
 }
 
@@ -897,7 +897,7 @@ static void zsolve_srk(const ZSolveArgs<float>& a, cudaStream_t s, cudaStream_t 
     cudaEventRecord(fork, s);
     cudaStreamWaitEvent(side, fork, 0);
     const size_t smem = (((size_t)a.g.NZ * 24 + 31) & ~(size_t)31) + (size_t)a.g.NZ * sizeof(cplx<double>);
-    cudaFuncSetAttribute(k_zsolve_srk_low, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    smem_limit(k_zsolve_srk_low, smem);
     k_zsolve_srk_low<<<a.g.low_modes * (2 * a.g.low_modes - 1), 128, smem, side>>>(a);
     cudaEventRecord(join, side);
     const size_t MH = (size_t)a.g.NXH * (a.g.NY / 2 + 1);

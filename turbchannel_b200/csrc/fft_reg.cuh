@@ -166,6 +166,7 @@ TC_FFT_SPLIT(972, 27, 36)
 TC_FFT_SPLIT(1024, 32, 32)
 #undef TC_FFT_SPLIT
 
+// a twiddle factor (a table that no kernel writes: read-only loads)
 template <typename T>
 __device__ __forceinline__ cplx<T> ldg_c(const cplx<T>* p) {
     if constexpr (sizeof(T) == 4) {

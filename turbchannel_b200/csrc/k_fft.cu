@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 3 : 4) k_div_quad_z(DivF
         T e[9];  // u at x-1 .. x+7
         {
             const Acc4<T> U0 = ld4(u + id), U1 = ld4(u + rb + xq);
-            e[0] = __ldg(u + rb + xm);
+            e[0] = u[rb + xm];
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 e[1 + k] = U0.v[k];

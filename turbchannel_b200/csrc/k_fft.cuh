@@ -89,7 +89,7 @@ __host__ __device__ constexpr bool xfft_alias(int rows) {
 
 // Three CTAs per SM in float (79 registers at N = 384, no spill), two in double.
 template <typename T, int N>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_xfft_reg(DivFftArgs<T> a, const T* __restrict__ src, int rows, unsigned mrows) {
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_xfft_reg(DivFftArgs<T> a, const T* src, int rows, unsigned mrows) {
     constexpr int N1 = FftSplit<N>::N1, N2 = FftSplit<N>::N2, YL = FftSplit<N>::YL, ZS = N + 1;
     extern __shared__ __align__(16) unsigned char smraw[];
     const Geom& g = a.g;
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_xfft_reg(DivFft
         const T* d0 = plane + (size_t)(2 * l) * N + n2;
         cplx<T> v[N1];
 #pragma unroll
-        for (int n1 = 0; n1 < N1; n1++) v[n1] = {__ldg(d0 + n1 * N2), __ldg(d0 + N + n1 * N2)};
+        for (int n1 = 0; n1 < N1; n1++) v[n1] = {d0[n1 * N2], d0[N + n1 * N2]};
         fft_pass_a<T, N, -1>(v, n2, a.twx, Y + l * YL);
     }
     __syncthreads();

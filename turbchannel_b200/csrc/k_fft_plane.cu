@@ -60,7 +60,7 @@ struct PlaneFft {
 
 // One forward plane: rows of the real field src[z][y][x] -> spec[z][kx][ky].
 template <typename T, int NX, int NY>
-__global__ void __launch_bounds__(PF_NT) k_xyfft_plane(const T* __restrict__ src, cplx<T>* __restrict__ spec,
+__global__ void __launch_bounds__(PF_NT) k_xyfft_plane(const T* src, cplx<T>* __restrict__ spec,
                                                         const cplx<T>* __restrict__ twx,
                                                         const cplx<T>* __restrict__ twy) {
     using P = PlaneFft<T, NX, NY>;
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(PF_NT) k_xyfft_plane(const T* __restrict__ src
             const T* d0 = rows + (size_t)(b + 2 * l) * NX + n2;
             cplx<T> v[X1];
 #pragma unroll
-            for (int n1 = 0; n1 < X1; n1++) v[n1] = {__ldg(d0 + n1 * X2), __ldg(d0 + NX + n1 * X2)};
+            for (int n1 = 0; n1 < X1; n1++) v[n1] = {d0[n1 * X2], d0[NX + n1 * X2]};
             fft_pass_a<T, NX, -1>(v, n2, twx, Y + l * XYL);
         }
         __syncthreads();
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(PF_NT) k_xyfft_plane(const T* __restrict__ src
 
 // One inverse plane: spec[z][kx][ky] -> p[z][y][x] * scale.
 template <typename T, int NX, int NY>
-__global__ void __launch_bounds__(PF_NT) k_ixyfft_plane(const cplx<T>* __restrict__ spec, T* __restrict__ p,
+__global__ void __launch_bounds__(PF_NT) k_ixyfft_plane(const cplx<T>* spec, T* __restrict__ p,
                                                          const cplx<T>* __restrict__ twx,
                                                          const cplx<T>* __restrict__ twy, T scale) {
     using P = PlaneFft<T, NX, NY>;
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(PF_NT) k_ixyfft_plane(const cplx<T>* __restric
             const cplx<T>* srcl = spec + ((size_t)z * NXH + kx) * NY + n2;
             cplx<T> v[Y1];
 #pragma unroll
-            for (int n1 = 0; n1 < Y1; n1++) v[n1] = ldg_c(srcl + n1 * Y2);
+            for (int n1 = 0; n1 < Y1; n1++) v[n1] = srcl[n1 * Y2];
             fft_pass_a<T, NY, +1>(v, n2, twy, Y + l * YYL);
         }
         __syncthreads();

@@ -150,22 +150,22 @@ __global__ void __launch_bounds__(STX* STY, coll_ctas<T, VISC, ORDER>()) k_flux_
             if (ORDER >= 2) {
 #pragma unroll
                 for (int c = 0; c < 3; c++) {
-                    hp[q][c] = __ldg(a.fp.c[c] + id);
+                    hp[q][c] = a.fp.c[c][id];
                     if (ORDER == 3) {
-                        hq[q][c] = __ldg(a.fq.c[c] + id);
-                        vq[q][c] = __ldg(a.velq.c[c] + id);
+                        hq[q][c] = a.fq.c[c][id];
+                        vq[q][c] = a.velq.c[c][id];
                     }
                 }
             }
             if (STAB1 && ORDER > 0 && !wall) {
                 const T* p = a.pcur + (size_t)z * NXY;
                 const int ym = wrapi(iy - 1, NY), yp = wrapi(iy + 1, NY);
-                pn[q][0] = __ldg(p + (size_t)iy * NX + xp);
-                pn[q][1] = __ldg(p + (size_t)iy * NX + xm);
-                pn[q][2] = __ldg(p + (size_t)yp * NX + ix);
-                pn[q][3] = __ldg(p + (size_t)ym * NX + ix);
-                pn[q][4] = __ldg(a.pcur + id + NXY);
-                pn[q][5] = __ldg(a.pcur + id - NXY);
+                pn[q][0] = p[(size_t)iy * NX + xp];
+                pn[q][1] = p[(size_t)iy * NX + xm];
+                pn[q][2] = p[(size_t)yp * NX + ix];
+                pn[q][3] = p[(size_t)ym * NX + ix];
+                pn[q][4] = a.pcur[id + NXY];
+                pn[q][5] = a.pcur[id - NXY];
             }
         }
         cp_async_wait<1>();
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(STX* STY, coll_ctas<T, VISC, ORDER>()) k_flux_
                     auto nut = [&](int ex, int ey, int ez) -> T {
                         if (!LES) return T(0);
                         const int xx = ex < 0 ? xm : ix, yy = ey < 0 ? ym : iy;
-                        return __ldg(a.nu_t + (size_t)(z + ez) * NXY + (size_t)yy * NX + xx);
+                        return ld_here(a.nu_t + (size_t)(z + ez) * NXY + (size_t)yy * NX + xx);
                     };
                     T gv[3];
                     visc_galerkin(A, nut, z, cDZ, hx, hy, ihx, ihy, visc, gv);

@@ -100,7 +100,7 @@ struct TileCopyX2 {
     }
 };
 
-__device__ __forceinline__ F2 ld2(const float* p) { return F2(__ldg(reinterpret_cast<const float2*>(p))); }
+__device__ __forceinline__ F2 ld2(const float* p) { return F2(*reinterpret_cast<const float2*>(p)); }
 __device__ __forceinline__ void st2(float* p, F2 v) { *reinterpret_cast<float2*>(p) = v.v; }
 __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { return F2(__ffma2_rn(a.v, b.v, c.v)); }
 

@@ -36,7 +36,7 @@ __device__ __forceinline__ void flux_cell(const RingAcc<T, SCHEME == TC_SCHEME_V
             if (!LES) return visc;
             const int xx = dx < 0 ? xm : (dx > 0 ? xp : ix);
             const int yy = dy < 0 ? ym : (dy > 0 ? yp : iy);
-            return visc + __ldg(nt + (size_t)(z + dz) * NXY + (size_t)yy * a.g.NX + xx);
+            return visc + ld_here(nt + (size_t)(z + dz) * NXY + (size_t)yy * a.g.NX + xx);
         };
         visc_naive<T, ACC, decltype(MU), INT>(A, MU, mz, vf);
     }
@@ -106,10 +106,10 @@ __global__ void __launch_bounds__(STX* TY, 2) k_flux_stag(FluxArgs<T> a, int tz)
                     const size_t id = (size_t)z * NXY + (size_t)iy * NX + ix;
 #pragma unroll
                     for (int c = 0; c < 3; c++) {
-                        hp[q][c] = __ldg(a.fp.c[c] + id);
+                        hp[q][c] = a.fp.c[c][id];
                         if (ORDER == 3) {
-                            hq[q][c] = __ldg(a.fq.c[c] + id);
-                            vq[q][c] = __ldg(a.velq.c[c] + id);
+                            hq[q][c] = a.fq.c[c][id];
+                            vq[q][c] = a.velq.c[c][id];
                         } else {
                             hq[q][c] = vq[q][c] = T(0);
                         }

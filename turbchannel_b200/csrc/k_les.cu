@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(128, 4) k_turb_mlp(TurbArgs<T> a, const float*
                 const unsigned i00 = iy * NX + ix, i10 = iy * NX + xp, i01 = yp * NX + ix, i11 = yp * NX + xp;
 #pragma unroll
                 for (int cc = 0; cc < 3; cc++) {
-                    const T* __restrict__ q = a.v.c[cc];
+                    const T* q = a.v.c[cc];
                     const T q000 = q[p0 + i00], q100 = q[p0 + i10], q010 = q[p0 + i01], q110 = q[p0 + i11];
                     const T q001 = q[p1 + i00], q101 = q[p1 + i10], q011 = q[p1 + i01], q111 = q[p1 + i11];
                     G[cc][0] = (float)((q100 + q110 + q101 + q111) - (q000 + q010 + q001 + q011)) * gx;
@@ -213,9 +213,9 @@ __global__ void __launch_bounds__(128, 4) k_turb_mlp(TurbArgs<T> a, const float*
                     G[cc][2] = (float)((q001 + q101 + q011 + q111) - (q000 + q100 + q010 + q110)) * gz;
                 }
             } else {
-                const T* __restrict__ u = a.v.c[0];
-                const T* __restrict__ v = a.v.c[1];
-                const T* __restrict__ w = a.v.c[2];
+                const T* u = a.v.c[0];
+                const T* v = a.v.c[1];
+                const T* w = a.v.c[2];
                 const unsigned xm = ix == 0 ? NX - 1u : ix - 1u, xpp = (int)xp + 1 == NX ? 0u : xp + 1u;
                 const unsigned ym = iy == 0 ? NY - 1u : iy - 1u, ypp = (int)yp + 1 == NY ? 0u : yp + 1u;
                 const unsigned pl = iz * NXY;

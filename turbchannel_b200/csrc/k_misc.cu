@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(KX* KY) k_correct(CorrArgs<T> a, int tz) {
     const int zb = blockIdx.z * ZC;
     const int xm = wrapi(ix - 1, NX), xmm = wrapi(ix - 2, NX), xp = wrapi(ix + 1, NX);
     const int ym = wrapi(iy - 1, NY), ymm = wrapi(iy - 2, NY), yp = wrapi(iy + 1, NY);
-    const T* __restrict__ p = a.p;
+    const T* p = a.p;
     T du = 0;
     if (!GRADONLY && a.cfr) {
         const double ub = (*a.ub_sum) * a.cfr_scale * (double)a.tob;
@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(KX* KY) k_correct(CorrArgs<T> a, int tz) {
 #pragma unroll
     for (int k = 0; k < ZC + 3; k++) {
         const int z = zb - 2 + k;
-        col[k] = (z >= 0 && z < NZ) ? __ldg(p + (size_t)z * NXY + (size_t)iy * NX + ix) : T(0);
+        col[k] = (z >= 0 && z < NZ) ? p[(size_t)z * NXY + (size_t)iy * NX + ix] : T(0);
     }
     T nb[ZC][6], rh[ZC][3], pc[ZC];
 #pragma unroll
@@ -85,17 +85,17 @@ __global__ void __launch_bounds__(KX* KY) k_correct(CorrArgs<T> a, int tz) {
         const int z = zb + k;
         if (z >= NZ) break;
         const size_t pl = (size_t)z * NXY;
-        nb[k][0] = __ldg(p + pl + (size_t)iy * NX + xm);
-        nb[k][1] = __ldg(p + pl + (size_t)iy * NX + xmm);
-        nb[k][2] = __ldg(p + pl + (size_t)iy * NX + xp);
-        nb[k][3] = __ldg(p + pl + (size_t)ym * NX + ix);
-        nb[k][4] = __ldg(p + pl + (size_t)ymm * NX + ix);
-        nb[k][5] = __ldg(p + pl + (size_t)yp * NX + ix);
+        nb[k][0] = p[pl + (size_t)iy * NX + xm];
+        nb[k][1] = p[pl + (size_t)iy * NX + xmm];
+        nb[k][2] = p[pl + (size_t)iy * NX + xp];
+        nb[k][3] = p[pl + (size_t)ym * NX + ix];
+        nb[k][4] = p[pl + (size_t)ymm * NX + ix];
+        nb[k][5] = p[pl + (size_t)yp * NX + ix];
         if (!GRADONLY) {
             const size_t id = pl + (size_t)iy * NX + ix;
 #pragma unroll
-            for (int c = 0; c < 3; c++) rh[k][c] = __ldg(a.rhs.c[c] + id);
-            if (STAB1) pc[k] = __ldg(a.pcur + id);
+            for (int c = 0; c < 3; c++) rh[k][c] = a.rhs.c[c][id];
+            if (STAB1) pc[k] = a.pcur[id];
         }
     }
 #pragma unroll
@@ -142,6 +142,9 @@ constexpr int correct_quad_planes() { return sizeof(T) == 4 ? 2 : 1; }
 template <typename T, int SCHEME, bool STAB1>
 __global__ void __launch_bounds__(QX* QY, 3) k_correct_quad(CorrArgs<T> a) {
     constexpr int ZN = correct_quad_planes<T>();
+    // the right-hand side loaded after the gradient, which otherwise spills: VV4 FP64 384x384x256
+    // 0.348 ms against 0.358 with every load ahead, collocated FP64 256x256x192 0.117 against 0.123
+    constexpr bool LATE = sizeof(T) == 8 && SCHEME != TC_SCHEME_HW2;
     const Geom& g = a.g;
     pdl_launch();
     pdl_wait();
@@ -155,7 +158,7 @@ __global__ void __launch_bounds__(QX* QY, 3) k_correct_quad(CorrArgs<T> a) {
     const int x = 4 * xq, zb = (sizeof(T) == 4 ? (int)(gridDim.z - 1 - blockIdx.z) : (int)blockIdx.z) * ZN;
     const int xl = x == 0 ? NX - 4 : x - 4, xr = x + 4 == NX ? 0 : x + 4;
     const int ym = wrapi(iy - 1, NY), ymm = wrapi(iy - 2, NY), yp = wrapi(iy + 1, NY);
-    const T* __restrict__ p = a.p;
+    const T* p = a.p;
     T du = 0;
     if (a.cfr) {
         const double ub = (*a.ub_sum) * a.cfr_scale * (double)a.tob;
@@ -185,9 +188,11 @@ __global__ void __launch_bounds__(QX* QY, 3) k_correct_quad(CorrArgs<T> a) {
         pym[k] = ld4(p + pl + (size_t)ym * NX + x);
         pymm[k] = ld4(p + pl + (size_t)ymm * NX + x);
         pyp[k] = ld4(p + pl + (size_t)yp * NX + x);
+        if constexpr (!LATE) {
 #pragma unroll
-        for (int c = 0; c < 3; c++) rh[k][c] = ld4(a.rhs.c[c] + pl + row + x);
-        if (STAB1) pc[k] = ld4(a.pcur + pl + row + x);
+            for (int c = 0; c < 3; c++) rh[k][c] = ld4(a.rhs.c[c] + pl + row + x);
+            if (STAB1) pc[k] = ld4(a.pcur + pl + row + x);
+        }
     }
 #pragma unroll
     for (int k = 0; k < ZN; k++) {
@@ -201,14 +206,20 @@ __global__ void __launch_bounds__(QX* QY, 3) k_correct_quad(CorrArgs<T> a) {
             e[4 + j] = col[k + 2].v[j];
             e[8 + j] = pr4[k].v[j];
         }
-        T o[3][4], pn[4];
+        T gp[4][3], o[3][4], pn[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            grad_at<T, SCHEME>(a, z, NZ, e[4 + j], e[3 + j], e[2 + j], e[5 + j], pym[k].v[j], pymm[k].v[j], pyp[k].v[j],
+                               col[k + 1].v[j], col[k].v[j], col[k + 3].v[j], gp[j]);
+        if constexpr (LATE) {
+#pragma unroll
+            for (int c = 0; c < 3; c++) rh[k][c] = ld4_here(a.rhs.c[c] + id);
+            if (STAB1) pc[k] = ld4_here(a.pcur + id);
+        }
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            T gp[3];
-            grad_at<T, SCHEME>(a, z, NZ, e[4 + j], e[3 + j], e[2 + j], e[5 + j], pym[k].v[j], pymm[k].v[j], pyp[k].v[j],
-                               col[k + 1].v[j], col[k].v[j], col[k + 3].v[j], gp);
 #pragma unroll
-            for (int c = 0; c < 3; c++) o[c][j] = (rh[k][c].v[j] - gp[c]) * a.tob;
+            for (int c = 0; c < 3; c++) o[c][j] = (rh[k][c].v[j] - gp[j][c]) * a.tob;
             if (a.cfr && !(SCHEME == TC_SCHEME_COLLOC && (z == 0 || z == NZ - 1))) o[0][j] += du;
             if (STAB1) pn[j] = col[k + 2].v[j] + pc[k].v[j];
         }
@@ -284,7 +295,7 @@ struct GAcc {
         }
     }
     __device__ __forceinline__ T operator()(int c, int dx, int dy, int dz) const {
-        return __ldg(v[c] + base + (long long)dz * (long long)NXY + (y[dy + 1] + x[dx + 1]));
+        return v[c][base + (long long)dz * (long long)NXY + (y[dy + 1] + x[dx + 1])];
     }
 };
 
@@ -530,7 +541,7 @@ __global__ void __launch_bounds__(QX* QY) k_correct_diag(CorrArgs<T> a) {
     const int x = 4 * (act ? xq : 0), zb = blockIdx.z * ZN, yy = act ? iy : 0;
     const int xl = x == 0 ? NX - 4 : x - 4, xr = x + 4 == NX ? 0 : x + 4;
     const int ym = wrapi(yy - 1, NY), ymm = wrapi(yy - 2, NY), yp = wrapi(yy + 1, NY);
-    const T* __restrict__ p = a.p;
+    const T* p = a.p;
     T du = 0;
     if (a.cfr) {
         const double ub = (*a.ub_sum) * a.cfr_scale * (double)a.tob;

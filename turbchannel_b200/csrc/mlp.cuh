@@ -43,7 +43,7 @@ struct alignas(16) MlpSmem {
 };
 
 // Fill from the packed FP32 parameters (cooperatively by the CTA; caller syncs).
-__device__ __forceinline__ void mlp_load_smem(MlpSmem& S, const float* __restrict__ P) {
+__device__ __forceinline__ void mlp_load_smem(MlpSmem& S, const float* P) {
     for (int e = threadIdx.x; e < MLP_H * MLP_K1; e += blockDim.x) {
         const int k = e / MLP_H, n = e - k * MLP_H;
         S.W1T[n][k] = __float2bfloat16_rn(k < MLP_IN ? P[MLP_OW1 + k * MLP_H + n] : 0.f);

@@ -20,31 +20,31 @@ __device__ __forceinline__ T div_at(const Geom& g, const MeshDev<T>& mesh, const
     const T ihx = (T)g.inv_hx, ihy = (T)g.inv_hy;
     if (SCHEME == TC_SCHEME_HW2) {
         const T hz = mesh.DZ[z];
-        return (__ldg(u + row + xp) - __ldg(u + id)) * ihx * hz +
-               (__ldg(v + (size_t)z * NXY + (size_t)yp * NX + x) - __ldg(v + id)) * ihy * hz +
-               ((z < NZ - 1) ? (__ldg(w + id + NXY) - __ldg(w + id)) : (-__ldg(w + id)));
+        return (u[row + xp] - u[id]) * ihx * hz +
+               (v[(size_t)z * NXY + (size_t)yp * NX + x] - v[id]) * ihy * hz +
+               ((z < NZ - 1) ? (w[id + NXY] - w[id]) : (-w[id]));
     } else if (SCHEME == TC_SCHEME_VV4) {
         const T C27 = T(0.03703703703703703703);
         const int xpp = xp + 1 == NX ? 0 : xp + 1, ypp = yp + 1 == NY ? 0 : yp + 1;
         const T dz = mesh.DZ[z], dzw = mesh.DZW[z];
-        const T dudx = ihx * (dz * (__ldg(u + row + xp) - __ldg(u + id)) - C27 * dzw * (__ldg(u + row + xpp) - __ldg(u + row + xm)));
+        const T dudx = ihx * (dz * (u[row + xp] - u[id]) - C27 * dzw * (u[row + xpp] - u[row + xm]));
         const size_t pl = (size_t)z * NXY;
-        const T dvdy = ihy * (dz * (__ldg(v + pl + (size_t)yp * NX + x) - __ldg(v + id)) -
-                              C27 * dzw * (__ldg(v + pl + (size_t)ypp * NX + x) - __ldg(v + pl + (size_t)ym * NX + x)));
-        const T w0 = __ldg(w + id);
-        const T wr = (z == NZ - 1) ? T(0) : __ldg(w + id + NXY);
-        const T wrr = (z == NZ - 1) ? w0 : (z == NZ - 2) ? T(0) : __ldg(w + id + 2 * NXY);
-        const T wll = (z == 0) ? __ldg(w + id + NXY) : (z == 1) ? T(0) : __ldg(w + id - NXY);
+        const T dvdy = ihy * (dz * (v[pl + (size_t)yp * NX + x] - v[id]) -
+                              C27 * dzw * (v[pl + (size_t)ypp * NX + x] - v[pl + (size_t)ym * NX + x]));
+        const T w0 = w[id];
+        const T wr = (z == NZ - 1) ? T(0) : w[id + NXY];
+        const T wrr = (z == NZ - 1) ? w0 : (z == NZ - 2) ? T(0) : w[id + 2 * NXY];
+        const T wll = (z == 0) ? w[id + NXY] : (z == 1) ? T(0) : w[id - NXY];
         return dudx + dvdy + (wr - w0) - C27 * (wrr - wll);
     } else {
         const T hz = mesh.cellh[z], hx = (T)g.hx, hy = (T)g.hy;
         const size_t pl = (size_t)z * NXY;
         T d = 0;
-        d += T(0.5) * (__ldg(u + row + xp) - __ldg(u + row + xm)) * hy * hz;
-        d += T(0.5) * (__ldg(v + pl + (size_t)yp * NX + x) - __ldg(v + pl + (size_t)ym * NX + x)) * hx * hz;
-        if (z == 0) d += T(0.5) * (__ldg(w + id + NXY) - __ldg(w + id)) * hx * hy;
-        else if (z == NZ - 1) d += T(0.5) * (__ldg(w + id) - __ldg(w + id - NXY)) * hx * hy;
-        else d += T(0.5) * (__ldg(w + id + NXY) - __ldg(w + id - NXY)) * hx * hy;
+        d += T(0.5) * (u[row + xp] - u[row + xm]) * hy * hz;
+        d += T(0.5) * (v[pl + (size_t)yp * NX + x] - v[pl + (size_t)ym * NX + x]) * hx * hz;
+        if (z == 0) d += T(0.5) * (w[id + NXY] - w[id]) * hx * hy;
+        else if (z == NZ - 1) d += T(0.5) * (w[id] - w[id - NXY]) * hx * hy;
+        else d += T(0.5) * (w[id + NXY] - w[id - NXY]) * hx * hy;
         return d;
     }
 }

@@ -77,7 +77,7 @@ struct alignas(2 * sizeof(T)) cplx {
     T x, y;
 };
 
-// four consecutive elements as one (float) or two (double) 16-byte read-only loads;
+// four consecutive elements as one (float) or two (double) 16-byte loads;
 // the address must be 16-byte aligned
 template <typename T>
 struct Acc4 {
@@ -87,11 +87,11 @@ template <typename T>
 __device__ __forceinline__ Acc4<T> ld4(const T* p) {
     Acc4<T> r;
     if constexpr (sizeof(T) == 4) {
-        const float4 q = __ldg(reinterpret_cast<const float4*>(p));
+        const float4 q = *reinterpret_cast<const float4*>(p);
         r.v[0] = q.x; r.v[1] = q.y; r.v[2] = q.z; r.v[3] = q.w;
     } else {
-        const double2 q0 = __ldg(reinterpret_cast<const double2*>(p));
-        const double2 q1 = __ldg(reinterpret_cast<const double2*>(p) + 1);
+        const double2 q0 = *reinterpret_cast<const double2*>(p);
+        const double2 q1 = reinterpret_cast<const double2*>(p)[1];
         r.v[0] = q0.x; r.v[1] = q0.y; r.v[2] = q1.x; r.v[3] = q1.y;
     }
     return r;
@@ -106,8 +106,11 @@ __host__ __device__ __forceinline__ cplx<T> cmul(cplx<T> a, cplx<T> b) {
 // Programmatic dependent launch: a kernel launched with launch_pdl may start while the
 // kernel before it in its stream still runs; pdl_wait returns once that kernel (and so all
 // before it, each of them waiting first) has completed and its writes are visible.  Only
-// constants and data no kernel writes may be touched before it.  pdl_launch lets the next
-// kernel start its own prologue.
+// constants and data no kernel writes may be touched before it.  After it, what the kernels
+// before have written is read with plain loads: a read-only load (__ldg, or through const
+// __restrict__) promises data that stay constant for the whole life of the reading kernel, which
+// here begins while they are still written, and nothing then has to hold it behind the wait.
+// pdl_launch lets the next kernel start its own prologue.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
@@ -145,6 +148,31 @@ template <typename K>
 static inline void smem_limit(K kern, size_t bytes, size_t most = SMEM_MOST) {
     if (bytes > 32 * 1024)
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes > most ? bytes : most));
+}
+
+// A plain load that stays where it is written: the compiler else gathers the loads of an unrolled
+// loop ahead of it, in registers that the loop needs.
+__device__ __forceinline__ float ld_here(const float* p) {
+    float r;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(r) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ double ld_here(const double* p) {
+    double r;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(r) : "l"(p));
+    return r;
+}
+
+template <typename T>
+__device__ __forceinline__ Acc4<T> ld4_here(const T* p) {
+    Acc4<T> r;
+    if constexpr (sizeof(T) == 4)
+        asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]) : "l"(p));
+    else {
+        asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(r.v[0]), "=d"(r.v[1]) : "l"(p));
+        asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(r.v[2]), "=d"(r.v[3]) : "l"(p + 2));
+    }
+    return r;
 }
 
 // ---------------------------------------------------------------------------

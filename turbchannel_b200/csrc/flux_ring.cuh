@@ -10,6 +10,9 @@
 
 namespace tc {
 
+// planes per CTA of the collocated kernel, at most: those whose constants it keeps
+constexpr int CPLANES = 128;
+
 // Planes per CTA of a kernel with `tiles` tiles per plane and `ctas` CTAs per SM: one
 // wave of CTAs where the tiles leave room for it -- every further one refills its ring and
 // ends in a partly empty wave (8 chunks per SM before: VV4 FP64 192x192x96 216 -> 188 us,

@@ -14,7 +14,6 @@
 
 namespace tc {
 
-constexpr int CPLANES = 128;  // planes whose constants a CTA keeps in shared memory
 
 // Galerkin viscous term, collocated_AB3/func_fluxes.h:21-85 (without the final
 // 1/(hx hy hz) factor).  NUT(ex, ey, ez) = nu_t of the element with lower corner at
@@ -123,7 +122,7 @@ __global__ void __launch_bounds__(STX* STY, coll_ctas<T, VISC, ORDER>()) k_flux_
     // visc inv_hz / DZ[z], visc inv_hz / DZ[z-1] (cross viscosity); the per-node work
     // then has no double arithmetic
     __shared__ T pc[3][CPLANES];
-    for (int k = threadIdx.x; k < ze - zb && k < CPLANES; k += blockDim.x) {
+    for (int k = threadIdx.x; k < ze - zb; k += blockDim.x) {
         const int z = zb + k;
         if (z == 0 || z == NZ - 1) {
             pc[0][k] = pc[1][k] = pc[2][k] = T(0);
@@ -171,7 +170,7 @@ __global__ void __launch_bounds__(STX* STY, coll_ctas<T, VISC, ORDER>()) k_flux_
         cp_async_wait<1>();
         __syncthreads();
         const int kz = z - zb;
-        const T inv_hz = wall ? T(0) : (kz < CPLANES ? pc[0][kz] : (T)(2. / (cDZ[z - 1] + cDZ[z])));
+        const T inv_hz = pc[0][kz];  // 0 at a wall
         ACC A0;
         A0.set(ring, z & (RS - 1), tx, tyt * CY);
 #pragma unroll
@@ -213,10 +212,7 @@ __global__ void __launch_bounds__(STX* STY, coll_ctas<T, VISC, ORDER>()) k_flux_
                         const T u0 = A(c, 0, 0, 0);
                         f[c] += visc * ihx * ihx * (A(c, 1, 0, 0) + A(c, -1, 0, 0) - T(2.) * u0);
                         f[c] += visc * ihy * ihy * (A(c, 0, 1, 0) + A(c, 0, -1, 0) - T(2.) * u0);
-                        if (kz < CPLANES)
-                            f[c] += pc[1][kz] * (A(c, 0, 0, 1) - u0) - pc[2][kz] * (u0 - A(c, 0, 0, -1));
-                        else
-                            f[c] += visc * (T)(((double)A(c, 0, 0, 1) - u0) / cDZ[z] - ((double)u0 - A(c, 0, 0, -1)) / cDZ[z - 1]) * inv_hz;
+                        f[c] += pc[1][kz] * (A(c, 0, 0, 1) - u0) - pc[2][kz] * (u0 - A(c, 0, 0, -1));
                     }
                 }
                 f[0] += (T)g.sour_dpdx;
@@ -260,6 +256,10 @@ static void flux_coll_shape(const Geom& g, int cy, int ctas, dim3& grid, int& tz
     const int ty = STY * cy;
     const int tiles = ((g.NX + STX - 1) / STX) * ((g.NY + ty - 1) / ty);
     tz = flux_chunk(tiles, g.NZ, ctas);
+    if (tz > CPLANES) {
+        const int n = (g.NZ + CPLANES - 1) / CPLANES;
+        tz = (g.NZ + n - 1) / n;
+    }
     grid = dim3((g.NX + STX - 1) / STX, (g.NY + ty - 1) / ty, (g.NZ + tz - 1) / tz);
 }
 

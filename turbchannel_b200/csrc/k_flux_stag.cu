@@ -189,8 +189,12 @@ static void flux_stag_shape(const Geom& g, int tile_rows, dim3& grid, int& tz) {
 }
 
 // upper bound of the flux kernels' grid sizes (sizes the partial-sum buffer): every kernel has
-// at most max(592, 1184 + tiles) CTAs (flux_chunk), the smallest tile being 32 x 8
-int flux_grid_blocks(const Geom& g) { return 2 * 1184 + ((g.NX + STX - 1) / STX) * ((g.NY + STY - 1) / STY); }
+// at most max(888, 1184 + tiles) CTAs (flux_chunk) or, collocated, tiles of chunks of CPLANES
+// planes, the smallest tile being 32 x 8
+int flux_grid_blocks(const Geom& g) {
+    const int tiles = ((g.NX + STX - 1) / STX) * ((g.NY + STY - 1) / STY);
+    return 2 * 1184 + tiles * (1 + (g.NZ + CPLANES - 1) / CPLANES);
+}
 
 template <typename T, int SCHEME, int VISC, bool LES, int ORDER>
 static void run(const FluxArgs<T>& a, cudaStream_t s) {

@@ -13,21 +13,24 @@ namespace tc {
 // planes per CTA of the collocated kernel, at most: those whose constants it keeps
 constexpr int CPLANES = 128;
 
-// Planes per CTA of a kernel with `tiles` tiles per plane and `ctas` CTAs per SM: one
-// wave of CTAs where the tiles leave room for it -- every further one refills its ring and
-// ends in a partly empty wave (8 chunks per SM before: VV4 FP64 192x192x96 216 -> 188 us,
-// 96x96x96 67 -> 56, 192x192x256 527 -> 477; HW2 LES 192x192x128 mixed 122 -> 111; collocated
-// 128x128x128 mixed 48 -> 40) -- or two waves of tall chunks where one would leave some SMs
-// with a single CTA (collocated 256x256x192 FP64, 256 tiles: one chunk 353 us, two 333,
-// eight per SM 344; at 96 and 128 planes one chunk is the faster); more tiles than that: 8
-// chunks per SM (384x384x256 FP64, 576 tiles).
-static inline int flux_chunk(int tiles, int NZ, int ctas = 2) {
+// Planes per CTA of a kernel with `tiles` tiles per plane and `ctas` CTAs per SM: one wave of
+// CTAs, or two of tall chunks, where whole chunks fill it to 85% -- every further chunk refills
+// its ring of planes -- and else 8 chunks per SM, whose last wave is a small part of the whole.
+// Step times, filled wave / 8 per SM: VV4 FP64 96x96x96 (36 tiles, 97% full) 116 / 123 us,
+// 192x192x96 (144, 97%) 343 / 365, collocated mixed 128x128x48 (32, 86%) 44 / 50.  A wave left
+// half empty costs more than the refills: VV4 FP64 216x216x128 (189 tiles of 296 slots) 778 / 650,
+// collocated FP64 256x192x128 (192 tiles) 542 / 404, mixed 324x216x128 (154) 635 / 403.
+// waves = false: the Galerkin viscosity, whose time is its arithmetic, takes 8 per SM at every
+// size (FP64 128x128x128, 64 tiles, 419 / 369; 256x256x192, 256 tiles, 2210 / 2022).
+static inline int flux_chunk(int tiles, int NZ, int ctas = 2, bool waves = true) {
     const int slots = 148 * ctas;
-    int nch;
-    if (tiles > slots) nch = (148 * 8 + tiles - 1) / tiles;
-    else if (2 * tiles > slots && NZ >= 160) nch = 2 * slots / tiles;
-    else nch = slots / tiles;
-    return std::max(4, (NZ + nch - 1) / nch);
+    const bool tall = 2 * tiles > slots && NZ >= 160;
+    for (int k = 0; k < 2 && waves && tiles <= slots; k++) {
+        const int w = tall ? 2 - k : 1 + k, n = w * slots / tiles, tz = std::max(4, (NZ + n - 1) / n);
+        if (20ll * tiles * ((NZ + tz - 1) / tz) >= 17ll * w * slots) return tz;
+    }
+    const int n = (148 * 8 + tiles - 1) / tiles;
+    return std::max(4, (NZ + n - 1) / n);
 }
 
 constexpr int STX = 32, STY = 8;  // threads per CTA: 32 x 8

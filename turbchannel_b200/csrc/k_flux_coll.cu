@@ -252,10 +252,10 @@ __global__ void __launch_bounds__(STX* STY, coll_ctas<T, VISC, ORDER>()) k_flux_
 template <typename T>
 constexpr int coll_cy() { return sizeof(T) == 4 ? 2 : 1; }
 
-static void flux_coll_shape(const Geom& g, int cy, int ctas, dim3& grid, int& tz) {
+static void flux_coll_shape(const Geom& g, int cy, int ctas, bool waves, dim3& grid, int& tz) {
     const int ty = STY * cy;
     const int tiles = ((g.NX + STX - 1) / STX) * ((g.NY + ty - 1) / ty);
-    tz = flux_chunk(tiles, g.NZ, ctas);
+    tz = flux_chunk(tiles, g.NZ, ctas, waves);
     if (tz > CPLANES) {
         const int n = (g.NZ + CPLANES - 1) / CPLANES;
         tz = (g.NZ + n - 1) / n;
@@ -272,7 +272,7 @@ static void run(const FluxArgs<T>& a, cudaStream_t s) {
     smem_limit(kern, smem);
     dim3 grid;
     int tz;
-    flux_coll_shape(a.g, CY, coll_ctas<T, VISC, ORDER>(), grid, tz);
+    flux_coll_shape(a.g, CY, coll_ctas<T, VISC, ORDER>(), VISC != TC_VISC_GALERKIN, grid, tz);
     launch_pdl(a.g.pdl, kern, grid, STX * STY, smem, s, a, tz);
 }
 

@@ -273,7 +273,7 @@ static void run(const FluxArgs<T>& a, cudaStream_t s) {
     dim3 grid;
     int tz;
     flux_coll_shape(a.g, CY, coll_ctas<T, VISC, ORDER>(), VISC != TC_VISC_GALERKIN, grid, tz);
-    launch_pdl(a.g.pdl, kern, grid, STX * STY, smem, s, a, tz);
+    launch_pdl(a.g.pdl_flux, kern, grid, STX * STY, smem, s, a, tz);
 }
 
 template <typename T, int VISC, bool LES>

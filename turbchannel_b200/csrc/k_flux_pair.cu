@@ -390,14 +390,14 @@ static void run_pair(const FluxArgs<float>& a, cudaStream_t s) {
     const bool tma = a.staging == 1 && a.g.NX % PCX == 0 && a.g.NY % PTR == 0 && ntx >= 3 && nty >= 3 &&
                      velocity_tensor_map<H>(a, &tm);
     if (!tma) {
-        launch_pdl(a.g.pdl, plain, dim3(ntx, nty, nzc), PTX * PTR / PAIR_RY, smem, s, a, tz, 0, 0, tiles * nzc, tm);
+        launch_pdl(a.g.pdl_flux, plain, dim3(ntx, nty, nzc), PTX * PTR / PAIR_RY, smem, s, a, tz, 0, 0, tiles * nzc, tm);
         return;
     }
     auto boxed = k_flux_pair<SCHEME, ORDER, PAIR_RY, true>;
     cudaFuncSetAttribute(boxed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const int ni = (ntx - 2) * (nty - 2) * nzc;
-    launch_pdl(a.g.pdl, boxed, dim3(ntx - 2, nty - 2, nzc), PTX * PTR / PAIR_RY, smem, s, a, tz, 1, 0, tiles * nzc, tm);
-    launch_pdl(a.g.pdl, plain, dim3(2 * ntx + 2 * (nty - 2), 1, nzc), PTX * PTR / PAIR_RY, smem, s, a, tz, 2, ni, tiles * nzc, tm);
+    launch_pdl(a.g.pdl_flux, boxed, dim3(ntx - 2, nty - 2, nzc), PTX * PTR / PAIR_RY, smem, s, a, tz, 1, 0, tiles * nzc, tm);
+    launch_pdl(a.g.pdl_flux, plain, dim3(2 * ntx + 2 * (nty - 2), 1, nzc), PTX * PTR / PAIR_RY, smem, s, a, tz, 2, ni, tiles * nzc, tm);
 }
 
 template <int SCHEME>

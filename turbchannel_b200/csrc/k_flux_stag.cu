@@ -208,7 +208,7 @@ static void run(const FluxArgs<T>& a, cudaStream_t s) {
     dim3 grid;
     int tz;
     flux_stag_shape(a.g, TY * CY, grid, tz);
-    launch_pdl(a.g.pdl, kern, grid, STX * TY, smem, s, a, tz);
+    launch_pdl(a.g.pdl_flux, kern, grid, STX * TY, smem, s, a, tz);
 }
 
 template <typename T, int SCHEME, int VISC, bool LES>

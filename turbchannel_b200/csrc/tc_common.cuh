@@ -11,7 +11,10 @@ namespace tc {
 // ---------------------------------------------------------------------------
 // Plain data passed to kernels by value
 // ---------------------------------------------------------------------------
-constexpr long long TC_PDL_BYTES = 48ll << 20;
+// bytes of a field up to which the step's kernels, and its flux kernel, start early (Geom::pdl),
+// by the size of a value: float, double
+constexpr long long tc_pdl_bytes(int eb) { return (eb == 4 ? 48ll : 32ll) << 20; }
+constexpr long long tc_pdl_flux_bytes(int eb) { return (eb == 4 ? 4ll : 2ll) << 20; }
 struct Geom {
     int NX, NY, NZ, NXY;
     long long N;  // cells (or nodes)
@@ -22,13 +25,17 @@ struct Geom {
     // (collocated_AB3/func_global.h:163-170), 1 shift sum(p vol) / area
     // (collocated_SRK/func_global.h:130-137)
     int norm_srk = 0;
-    // programmatic launches between the step's kernels: fields up to TC_PDL_BYTES.  There the
-    // gaps between kernels are a large part of the step (64x64x64 FP64 with diagnostics 83.5 ->
-    // 73.5 us, 216x108x95 mixed 185 -> 168, 128x64x49 SRK 283 -> 230; up to 192x192x128 and
-    // 256x192x128 FP64, 36 and 48 MB a field, 385 -> 373 and 489 -> 485).  On larger grids CTAs
-    // of the next kernel take room from the running one: 256x256x192 FP64 931 -> 955 us,
-    // 384x384x256 mixed 1.61 -> 1.67 ms, FP64 3.60 -> 4.05 ms.
-    bool pdl = false;
+    // Programmatic launches between the step's kernels (pdl), on grids where the gaps between
+    // them are a large part of the step; of its flux kernel (pdl_flux), on the smallest alone.
+    // The flux kernel is one wave of long CTAs, and the room that the kernel before leaves free
+    // as it ends would place them unevenly, two on some SMs and one or none on others.  Steps
+    // back to back in us, without / with every kernel / with all but the flux kernel: VV4 mixed
+    // 256x256x192 503 / 605 / 502, collocated FP64 256x192x128 392 / 474 / 391, HW2 FP64
+    // 192x128x128 210 / 234 / 202, VV4 mixed 256x192x64 150 / 133 / 133, HW2 FP64 64x64x64
+    // 45.2 / 41.9 / 43.0.  Above 32 MB a field in FP64 the others lose 1 to 2% as well, in the
+    // mixed form they gain 3% up to 48 MB.  On larger grids CTAs of the next kernel take room from
+    // the running one: 256x256x192 FP64 931 without, 955 with, 384x384x256 mixed 1.61 and 1.67 ms.
+    bool pdl = false, pdl_flux = false;
 };
 
 // Mesh-derived arrays (device pointers into one allocation).  Staggered arrays

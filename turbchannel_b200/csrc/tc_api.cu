@@ -506,7 +506,7 @@ extern "C" int tc_create(const tc_params* prm, const double* zz, tc_handle** out
     g.NXH = p.NX / 2 + 1;
     const int eb = p.precision == TC_FP64 ? 8 : 4;
     g.pdl = g.N * eb <= tc_pdl_bytes(eb);
-    g.pdl_flux = g.N * eb <= tc_pdl_flux_bytes(eb);
+    g.pdl_flux = g.N * eb <= TC_PDL_FLUX_BYTES;
     g.scheme = p.scheme; g.visc_type = p.visc_type; g.turb = p.turb_model; g.stab_type = p.stab_type; g.fd_mode = p.fd_mode;
     int lm = p.low_modes > 0 ? p.low_modes : 4;
     lm = std::min(lm, std::min(g.NXH, (p.NY + 1) / 2));

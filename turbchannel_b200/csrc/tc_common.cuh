@@ -11,10 +11,10 @@ namespace tc {
 // ---------------------------------------------------------------------------
 // Plain data passed to kernels by value
 // ---------------------------------------------------------------------------
-// bytes of a field up to which the step's kernels, and its flux kernel, start early (Geom::pdl),
-// by the size of a value: float, double
+// bytes of a field up to which the step's kernels (by the size of a value: float, double), and
+// its flux kernel, start early (Geom::pdl)
 constexpr long long tc_pdl_bytes(int eb) { return (eb == 4 ? 48ll : 32ll) << 20; }
-constexpr long long tc_pdl_flux_bytes(int eb) { return (eb == 4 ? 4ll : 2ll) << 20; }
+constexpr long long TC_PDL_FLUX_BYTES = 4ll << 20;
 struct Geom {
     int NX, NY, NZ, NXY;
     long long N;  // cells (or nodes)
@@ -32,7 +32,8 @@ struct Geom {
     // back to back in us, without / with every kernel / with all but the flux kernel: VV4 mixed
     // 256x256x192 503 / 605 / 502, collocated FP64 256x192x128 392 / 474 / 391, HW2 FP64
     // 192x128x128 210 / 234 / 202, VV4 mixed 256x192x64 150 / 133 / 133, HW2 FP64 64x64x64
-    // 45.2 / 41.9 / 43.0.  Above 32 MB a field in FP64 the others lose 1 to 2% as well, in the
+    // 45.2 / 41.9 / 43.0, SRK 128x64x49 FP64 with diagnostics 209 with every kernel, 212 with all
+    // but the explicit term.  Above 32 MB a field in FP64 the others lose 1 to 2% as well, in the
     // mixed form they gain 3% up to 48 MB.  On larger grids CTAs of the next kernel take room from
     // the running one: 256x256x192 FP64 931 without, 955 with, 384x384x256 mixed 1.61 and 1.67 ms.
     bool pdl = false, pdl_flux = false;

@@ -129,16 +129,15 @@ __device__ __forceinline__ float rcp_fast(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-// silu of two values with one reciprocal: 1/(1+a) = (1+b) / ((1+a)(1+b)), a = e^-z0, b = e^-z1.
-// Three special-function operations for two values instead of four, at an error of two more
-// roundings (float ulps, below the BF16 rounding that follows); a, b are held below 2^63 so
-// that the product stays finite (silu below z = -44 is then -z 2^-63 instead of less).
+// silu of two values, each with its own exponential and reciprocal as in silu (the training
+// pass), the rest in packed arithmetic.  One reciprocal of the product of both denominators put
+// two more roundings into each value, and a bound on the exponentials in place of the values
+// below z = -44.
 __device__ __forceinline__ float2 silu2(float z0, float z1) {
     const float L2E = 1.44269504088896340736f;
     const float2 t = __fmul2_rn(make_float2(z0, z1), make_float2(-L2E, -L2E));
-    const float2 d = __fadd2_rn(make_float2(ex2_fast(fminf(t.x, 63.f)), ex2_fast(fminf(t.y, 63.f))), make_float2(1.f, 1.f));
-    const float r = rcp_fast(d.x * d.y);
-    return __fmul2_rn(make_float2(z0, z1), __fmul2_rn(make_float2(r, r), make_float2(d.y, d.x)));
+    const float2 d = __fadd2_rn(make_float2(ex2_fast(t.x), ex2_fast(t.y)), make_float2(1.f, 1.f));
+    return __fmul2_rn(make_float2(z0, z1), make_float2(rcp_fast(d.x), rcp_fast(d.y)));
 }
 // B fragments of two k-steps (kk, kk+1) of n-tile nt from a [n][k] bf16 array in one ldmatrix.
 template <int LD>

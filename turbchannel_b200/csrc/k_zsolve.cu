@@ -27,7 +27,6 @@
 // thread per mode sweeping global memory from one wall to the other: its forward result
 // went out to L2/DRAM and came back (16 B more), each sweep read factors of its own (16 B
 // or 6 B), and small grids had too few threads to hide the load latency of each row batch.
-// Measured:
 // before -> now, us (before: the sweep, its double low modes next to it on a side stream):
 //   HW2 64x64x64 FP64 17.1 (+ 5.6) -> 5.5      HW2 128x128x128 FP64 34.0 (+ 8.8) -> 11.3
 //   coll 256x256x192 FP64 98 (+ 16) -> 61-65   VV4 216x108x95 mixed 17-24 (+ 9) -> 11.6
@@ -80,15 +79,32 @@ static int zs_pairs(const Geom& g, int eb) {
 }
 static int zs_pairs_low(const Geom& g) { return std::max(1, zs_pairs(g, 4) / 2); }  // double tiles of the mixed mode
 
-// VV4 grids in double with many modes keep one thread per mode sweeping global memory
-// (k_zsolve_stream): a tile's columns and factors take 64 KB per 4 pairs there, half the lanes
-// of each sweeping warp are idle and three tiles fit an SM, while the streaming form has
-// enough modes in flight to run at its DRAM traffic: streaming / tiles 0.187 / 0.192 ms at
-// 288x288x256, 0.211 / 0.244 at 324x324x256, 0.264 / 0.335 at 384x384x256, 0.089 / 0.093 at
-// 384x384x96; below 288x288 the tiles win (192x192x256: 0.088 against 0.120).
-constexpr long long ZS_STREAM_MODES = 42000;
+// Pairs of modes whose columns an SM holds at a time: 1 KB of the system's and the kernel's own
+// shared memory next to each tile.
+static int zs_resident_pairs(const Geom& g, int eb) {
+    const int kp = zs_pairs(g, eb);
+    return kp * (int)std::min<size_t>(32, 228 * 1024 / (zs_smem(g, kp, eb) + 2592));
+}
+
+// One thread per mode sweeping global memory (k_zsolve_stream) in place of tiles:
+// VV4 grids in double with many modes (288x288 and larger), where a tile's columns and factors
+// take 64 KB per 4 pairs, half the lanes of each sweeping warp are idle and three tiles fit an SM,
+// while the streaming form has enough modes in flight to run at its DRAM traffic: streaming /
+// tiles 0.187 / 0.192 ms at 288x288x256 (equal at 96 and 192 planes), 0.211 / 0.244 at
+// 324x324x256, 0.264 / 0.335 at 384x384x256, 0.089 / 0.093 at 384x384x96; below, the tiles win
+// (192x192x256: 0.088 against 0.120) or are equal (256x256x256).
+// And columns so long that an SM holds few pairs, in grids with the modes to fill the chip
+// another way (a spectrum beyond the L2, 150 MB): whole solves, streaming / tiles in us, HW2 FP64
+// 256x256x1024 (4 pairs per SM) 1360 / 1720, VV4 FP64 256x256x1024 (3) 1520 / 2570, mixed (6)
+// 830 / 1090, HW2 mixed 128x128x2800 (3) 850 / 1290; but HW2 FP64 128x128x700 (93 MB) 318 / 273,
+// and 256x256x384 (12 pairs) 513 / 529.
+constexpr long long ZS_STREAM_MODES = 41000, ZS_STREAM_BYTES = 150000000;
+constexpr int ZS_STREAM_PAIRS = 8;
 static bool zs_stream(const Geom& g, int eb) {
-    return eb == 8 && zs_vv(g) && (long long)g.NXH * g.NY >= ZS_STREAM_MODES;
+    if (eb == 4 && g.norm_srk != 0) return false;
+    const long long modes = (long long)g.NXH * g.NY;
+    if (eb == 8 && zs_vv(g) && modes >= ZS_STREAM_MODES) return true;
+    return modes * g.NZ * 2 * eb >= ZS_STREAM_BYTES && zs_resident_pairs(g, eb) <= ZS_STREAM_PAIRS;
 }
 
 // The mixed SRK step keeps the one-sided solve of one thread per mode (k_zsolve_srk): its
@@ -114,6 +130,7 @@ size_t zfactor_low_bytes(const Geom& g) {
 // ---------------------------------------------------------------------------
 template <typename T, int SCHEME>
 __global__ void __launch_bounds__(128) k_zfactor(ZSolveArgs<T> a, int kp, int kpl, bool stream) {
+    // tiles: a.fac and (the mixed mode) a.fac_low; stream: a.fac alone; a.fac null: a.fac_low alone
     constexpr bool VV = SCHEME == TC_SCHEME_VV4;
     constexpr int NV = VV ? 4 : 2;
     const Geom& g = a.g;
@@ -124,6 +141,7 @@ __global__ void __launch_bounds__(128) k_zfactor(ZSolveArgs<T> a, int kp, int kp
     const bool pin = (kx == 0 && ky == 0);
     const int LM = g.low_modes;
     const bool low = a.fac_low != nullptr && kx < LM && ky < LM;
+    if (a.fac == nullptr && !low) return;
     const int nkt = (NYH1 + kp - 1) / kp, nkl = (LM + kpl - 1) / kpl;
     // stream: eliminated from wall 0 to the far wall, [row][pair][value]
     const int top = stream ? NZ : zs_top(NZ, VV), half = zs_half(NZ, VV), rows = zs_rows(NZ, VV);
@@ -141,7 +159,7 @@ __global__ void __launch_bounds__(128) k_zfactor(ZSolveArgs<T> a, int kp, int kp
         const int i = row < top ? half - top + row
                                 : (row < top + zs_mid(VV) ? 2 * half + row - top
                                                          : 2 * half - (NZ - zs_mid(VV) - top) + NZ - 1 - row);
-        F[(size_t)i * kp * NV + v] = (T)x;
+        if (a.fac) F[(size_t)i * kp * NV + v] = (T)x;
         if (low) FL[(size_t)i * kpl * NV + v] = x;
     };
     // the row's diagonal and its coupling to row i + k
@@ -313,10 +331,17 @@ void launch_zfactor(const ZSolveArgs<T>& a, cudaStream_t s) {
     const int kp = zs_pairs(a.g, sizeof(T)), kpl = zs_pairs_low(a.g);
     ZSolveArgs<T> b = a;
     if (sizeof(T) == 8) b.fac_low = nullptr;  // FP64: the low modes are modes like any other
-    const bool st = zs_stream(a.g, sizeof(T));
-    if (a.g.scheme == TC_SCHEME_VV4) k_zfactor<T, TC_SCHEME_VV4><<<nb, 128, 0, s>>>(b, kp, kpl, st);
-    else if (a.g.scheme == TC_SCHEME_HW2) k_zfactor<T, TC_SCHEME_HW2><<<nb, 128, 0, s>>>(b, kp, kpl, st);
-    else k_zfactor<T, TC_SCHEME_COLLOC><<<nb, 128, 0, s>>>(b, kp, kpl, st);
+    const auto k = a.g.scheme == TC_SCHEME_VV4   ? k_zfactor<T, TC_SCHEME_VV4>
+                   : a.g.scheme == TC_SCHEME_HW2 ? k_zfactor<T, TC_SCHEME_HW2>
+                                                 : k_zfactor<T, TC_SCHEME_COLLOC>;
+    if (zs_stream(a.g, sizeof(T))) {
+        b.fac_low = nullptr;
+        k<<<nb, 128, 0, s>>>(b, kp, kpl, true);
+        if (sizeof(T) == 8) return;
+        b.fac_low = a.fac_low;
+        b.fac = nullptr;
+    }
+    k<<<nb, 128, 0, s>>>(b, kp, kpl, false);
 }
 
 // ---------------------------------------------------------------------------
@@ -605,32 +630,36 @@ __global__ void __launch_bounds__(ZS_NT) k_zsolve_col(ZSolveArgs<T> a, int nlow,
     zsolve_tile<T, T, VV, KP, FS, false>(a, smz, kx, k0, NYH1, sizeof(T) == 4 ? LM : 0, fac, reinterpret_cast<T*>(mid));
 }
 
+// low_only: the low modes' tiles of a mixed solve whose other modes stream
 template <typename T, bool VV, int KP, bool FS = true>
-static void zsolve_kp(const ZSolveArgs<T>& a, cudaStream_t s) {
+static void zsolve_kp(const ZSolveArgs<T>& a, cudaStream_t s, bool low_only) {
     constexpr int KPL = KP > 1 ? KP / 2 : 1;
     const Geom& g = a.g;
     const int nkt = zs_ktiles(g, KP);
     const int nkl = (g.low_modes + KPL - 1) / KPL, nlow = sizeof(T) == 4 ? g.low_modes * nkl : 0;
-    size_t smem = zs_smem(g, KP, sizeof(T), FS);
+    size_t smem = low_only ? 0 : zs_smem(g, KP, sizeof(T), FS);
     if (nlow) smem = std::max(smem, zs_smem(g, KPL, 8, FS));
     if constexpr (KP == 1 && FS) {
-        if (smem > ZS_SMEM_MAX) return zsolve_kp<T, VV, 1, false>(a, s);
+        if (smem > ZS_SMEM_MAX) return zsolve_kp<T, VV, 1, false>(a, s, low_only);
     }
     auto k = k_zsolve_col<T, VV, KP, FS>;
     smem_limit(k, smem, FS ? SMEM_MOST : SMEM_MOST + 2048);
-    launch_pdl(a.g.pdl, k, (unsigned)(nlow + (size_t)g.NXH * nkt), ZS_NT, smem, s, a, nlow, nkl, nkt);
+    const size_t n = low_only ? 0 : (size_t)g.NXH * nkt;
+    launch_pdl(a.g.pdl && !low_only, k, (unsigned)(nlow + n), ZS_NT, smem, s, a, nlow, nkl, nkt);
 }
 
 // ---------------------------------------------------------------------------
-// 7-diagonal solve in double, one thread per mode (zs_stream)
+// one thread per mode (zs_stream)
 // ---------------------------------------------------------------------------
 // Adjacent lanes take the modes (kx, kh), (kx, NY-kh), which share their factors.  Rows are
-// moved R at a time through two register batches, the next batch's loads in flight; R = 2
-// keeps 5 CTAs of 128 threads per SM, so that the ~74 k modes of a 384 x 384 plane run in
+// moved R at a time through two register batches, the next batch's loads in flight.  FP64 VV4:
+// R = 2 keeps 5 CTAs of 128 threads per SM, so that the ~74 k modes of a 384 x 384 plane run in
 // one wave (384x384x256: 4 rows 0.318 ms, 3 rows 0.296, 2 rows 0.27-0.29).
-__global__ void __launch_bounds__(128) k_zsolve_stream(ZSolveArgs<double> a) {
-    constexpr int R = 2;
-    using C = cplx<double>;
+template <typename T, bool VV>
+__global__ void __launch_bounds__(128) k_zsolve_stream(ZSolveArgs<T> a) {
+    constexpr int R = sizeof(T) == 8 ? (VV ? 2 : 4) : (VV ? 4 : 6);
+    using C = cplx<T>;
+    using Q = typename std::conditional<VV, Q4<T>, Q2<T>>::type;
     const Geom& g = a.g;
     pdl_launch();
     pdl_wait();
@@ -639,16 +668,17 @@ __global__ void __launch_bounds__(128) k_zsolve_stream(ZSolveArgs<double> a) {
     const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t mh = t >> 1;
     const int kx = (int)(mh / NYH1), kh = (int)(mh - (size_t)kx * NYH1);
-    const bool act = mh < MH && !((t & 1) && (kh == 0 || 2 * kh == NY));  // odd lanes: no partner mode
-    if (!act && blockIdx.x != 0) return;
-    const Q4<double>* F = reinterpret_cast<const Q4<double>*>(a.fac) + mh;
+    bool act = mh < MH && !((t & 1) && (kh == 0 || 2 * kh == NY));  // odd lanes: no partner mode
+    if (sizeof(T) == 4 && kx < g.low_modes && kh < g.low_modes) act = false;
+    if (!act && (sizeof(T) == 4 || blockIdx.x != 0)) return;
+    const Q* F = reinterpret_cast<const Q*>(a.fac) + mh;
     C* x = a.spec + (size_t)kx * NY + ((t & 1) ? NY - kh : kh);
     C ra[R], rb[R];
-    Q4<double> fa[R], fb[R];
+    Q fa[R], fb[R];
     if (act) {
         C y1 = {0, 0}, y2 = {0, 0}, y3 = {0, 0};
-        double b1 = 0, b2 = 0, b2p = 0, b3 = 0, b3p = 0, b3q = 0;
-        auto load = [&](int i0, C(&r)[R], Q4<double>(&f)[R]) {
+        T b1 = 0, b2 = 0, b2p = 0, b3 = 0, b3p = 0, b3q = 0;
+        auto load = [&](int i0, C(&r)[R], Q(&f)[R]) {
 #pragma unroll
             for (int k = 0; k < R; k++)
                 if (i0 + k < NZ) {
@@ -656,19 +686,24 @@ __global__ void __launch_bounds__(128) k_zsolve_stream(ZSolveArgs<double> a) {
                     f[k] = F[(size_t)(i0 + k) * MH];
                 }
         };
-        auto run = [&](int i0, const C(&r)[R], const Q4<double>(&f)[R]) {
+        auto run = [&](int i0, const C(&r)[R], const Q(&f)[R]) {
 #pragma unroll
             for (int k = 0; k < R; k++) {
                 if (i0 + k >= NZ) break;
-                C y;
-                y.x = r[k].x - b3q * y3.x - b2p * y2.x;
-                y.y = r[k].y - b3q * y3.y - b2p * y2.y;
+                C y = r[k];
+                if constexpr (VV) {
+                    y.x = y.x - b3q * y3.x - b2p * y2.x;
+                    y.y = y.y - b3q * y3.y - b2p * y2.y;
+                    y3 = y2; y2 = y1;
+                }
                 y.x -= b1 * y1.x;
                 y.y -= b1 * y1.y;
                 x[(size_t)(i0 + k) * M] = y;
-                y3 = y2; y2 = y1; y1 = y;
-                b3q = b3p; b3p = b3; b3 = f[k].w;
-                b2p = b2; b2 = f[k].z;
+                y1 = y;
+                if constexpr (VV) {
+                    b3q = b3p; b3p = b3; b3 = f[k].w;
+                    b2p = b2; b2 = f[k].z;
+                }
                 b1 = f[k].y;
             }
         };
@@ -682,7 +717,7 @@ __global__ void __launch_bounds__(128) k_zsolve_stream(ZSolveArgs<double> a) {
     }
     if (act) {
         C x1 = {0, 0}, x2 = {0, 0}, x3 = {0, 0};
-        auto load = [&](int i0, C(&r)[R], Q4<double>(&f)[R]) {
+        auto load = [&](int i0, C(&r)[R], Q(&f)[R]) {
 #pragma unroll
             for (int k = 0; k < R; k++)
                 if (i0 - k >= 0) {
@@ -690,17 +725,22 @@ __global__ void __launch_bounds__(128) k_zsolve_stream(ZSolveArgs<double> a) {
                     f[k] = F[(size_t)(i0 - k) * MH];
                 }
         };
-        auto run = [&](int i0, const C(&r)[R], const Q4<double>(&f)[R]) {
+        auto run = [&](int i0, const C(&r)[R], const Q(&f)[R]) {
 #pragma unroll
             for (int k = 0; k < R; k++) {
                 if (i0 - k < 0) break;
                 C v;
-                v.x = r[k].x * f[k].x - f[k].w * x3.x - f[k].z * x2.x;
-                v.y = r[k].y * f[k].x - f[k].w * x3.y - f[k].z * x2.y;
+                v.x = r[k].x * f[k].x;
+                v.y = r[k].y * f[k].x;
+                if constexpr (VV) {
+                    v.x = v.x - f[k].w * x3.x - f[k].z * x2.x;
+                    v.y = v.y - f[k].w * x3.y - f[k].z * x2.y;
+                    x3 = x2; x2 = x1;
+                }
                 v.x -= f[k].y * x1.x;
                 v.y -= f[k].y * x1.y;
                 x[(size_t)(i0 - k) * M] = v;
-                x3 = x2; x2 = x1; x1 = v;
+                x1 = v;
             }
         };
         load(NZ - 1, ra, fa);
@@ -711,7 +751,7 @@ __global__ void __launch_bounds__(128) k_zsolve_stream(ZSolveArgs<double> a) {
             run(i0 - R, rb, fb);
         }
     }
-    if (blockIdx.x == 0) {  // mode (0, 0) is thread 0's
+    if (sizeof(T) == 8 && blockIdx.x == 0) {  // mode (0, 0) is thread 0's
         __shared__ double red[4];
         __syncthreads();
         auto row = [&](int i) { return (size_t)i * M; };
@@ -906,13 +946,35 @@ static void zsolve_srk(const ZSolveArgs<float>& a, cudaStream_t s, cudaStream_t 
 }
 
 template <typename T, bool VV>
-static void zsolve_vv(const ZSolveArgs<T>& a, cudaStream_t s) {
+static void zsolve_tiles(const ZSolveArgs<T>& a, cudaStream_t s, bool low_only) {
     switch (zs_pairs(a.g, sizeof(T))) {
-        case 8: zsolve_kp<T, VV, 8>(a, s); break;
-        case 4: zsolve_kp<T, VV, 4>(a, s); break;
-        case 2: zsolve_kp<T, VV, 2>(a, s); break;
-        default: zsolve_kp<T, VV, 1>(a, s); break;
+        case 8: zsolve_kp<T, VV, 8>(a, s, low_only); break;
+        case 4: zsolve_kp<T, VV, 4>(a, s, low_only); break;
+        case 2: zsolve_kp<T, VV, 2>(a, s, low_only); break;
+        default: zsolve_kp<T, VV, 1>(a, s, low_only); break;
     }
+}
+
+// returns launches
+template <typename T, bool VV>
+static int zsolve_vv(const ZSolveArgs<T>& a, cudaStream_t s, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join) {
+    if (!zs_stream(a.g, sizeof(T))) {
+        zsolve_tiles<T, VV>(a, s, false);
+        return 1;
+    }
+    const size_t n = (size_t)2 * a.g.NXH * (a.g.NY / 2 + 1);
+    if (sizeof(T) == 8) {
+        launch_pdl(a.g.pdl, k_zsolve_stream<T, VV>, (unsigned)((n + 127) / 128), 128, 0, s, a);
+        return 1;
+    }
+    // the two sets of modes are disjoint: the low modes' tiles on the side stream
+    cudaEventRecord(fork, s);
+    cudaStreamWaitEvent(side, fork, 0);
+    zsolve_tiles<T, VV>(a, side, true);
+    cudaEventRecord(join, side);
+    launch_pdl(false, k_zsolve_stream<T, VV>, (unsigned)((n + 127) / 128), 128, 0, s, a);
+    cudaStreamWaitEvent(s, join, 0);
+    return 2;
 }
 
 template <typename T>
@@ -923,16 +985,7 @@ int launch_zsolve_fac(const ZSolveArgs<T>& a, cudaStream_t s, cudaStream_t side,
             return 2;
         }
     }
-    if constexpr (sizeof(T) == 8) {
-        if (zs_stream(a.g, sizeof(T))) {
-            const size_t n = (size_t)2 * a.g.NXH * (a.g.NY / 2 + 1);
-            launch_pdl(a.g.pdl, k_zsolve_stream, (unsigned)((n + 127) / 128), 128, 0, s, a);
-            return 1;
-        }
-    }
-    if (a.g.scheme == TC_SCHEME_VV4) zsolve_vv<T, true>(a, s);
-    else zsolve_vv<T, false>(a, s);
-    return 1;
+    return a.g.scheme == TC_SCHEME_VV4 ? zsolve_vv<T, true>(a, s, side, fork, join) : zsolve_vv<T, false>(a, s, side, fork, join);
 }
 
 template int launch_zsolve_fac<double>(const ZSolveArgs<double>&, cudaStream_t, cudaStream_t, cudaEvent_t, cudaEvent_t);

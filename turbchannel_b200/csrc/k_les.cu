@@ -173,9 +173,9 @@ __global__ void __launch_bounds__(256) k_les_features(const float* __restrict__ 
 // Smagorinsky kernel), with the element gradient of the nodal velocity -- the network's
 // inputs are invariants of the resolved gradient in wall units and y+, the same physical
 // quantities for both schemes.
-// Bound by instruction issue and the special-function unit: 128 SiLU per cell at 1.5
-// operations each are 24 us of that unit at 96x96x64 mixed, where the kernel takes 58 us (106 with
-// 16-sample tiles, two operations per SiLU, 64-bit index divisions and the full 3 x 3 products).
+// Bound by the special-function unit and instruction issue: 128 SiLU per cell at two operations
+// each are 32 us of that unit at 96x96x64 mixed, where the kernel takes 64 us (106 with 16-sample
+// tiles, 64-bit index divisions and the full 3 x 3 products).
 template <typename T, bool COLL>
 __global__ void __launch_bounds__(128, 4) k_turb_mlp(TurbArgs<T> a, const float* __restrict__ P) {
     __shared__ MlpSmem S;

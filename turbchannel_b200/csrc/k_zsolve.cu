@@ -95,16 +95,20 @@ static int zs_resident_pairs(const Geom& g, int eb) {
 // (192x192x256: 0.088 against 0.120) or are equal (256x256x256).
 // And columns so long that an SM holds few pairs, in grids with the modes to fill the chip
 // another way (a spectrum beyond the L2, 150 MB): whole solves, streaming / tiles in us, HW2 FP64
-// 256x256x1024 (4 pairs per SM) 1360 / 1720, VV4 FP64 256x256x1024 (3) 1520 / 2570, mixed (6)
-// 830 / 1090, HW2 mixed 128x128x2800 (3) 850 / 1290; but HW2 FP64 128x128x700 (93 MB) 318 / 273,
-// and 256x256x384 (12 pairs) 513 / 529.
-constexpr long long ZS_STREAM_MODES = 41000, ZS_STREAM_BYTES = 150000000;
+// 256x256x1024 (4 pairs per SM) 1300 / 1720, VV4 FP64 256x256x1024 (3) 1520 / 2570, mixed (6)
+// 790 / 1090, HW2 mixed 128x128x2800 (3) 780 / 1290; but HW2 FP64 128x128x700 (93 MB) 318 / 273
+// (4 rows per batch), and 256x256x384 (12 pairs) 513 / 529.  The mixed form streams from 100 MB on
+// where an SM holds 3 pairs or fewer: VV4 128x128x2048 (136 MB) 580 / 1081, HW2 96x96x2800 (104 MB)
+// 640 / 771.
+constexpr long long ZS_STREAM_MODES = 41000, ZS_STREAM_BYTES = 150000000, ZS_STREAM_BYTES_FEW = 100000000;
 constexpr int ZS_STREAM_PAIRS = 8;
 static bool zs_stream(const Geom& g, int eb) {
     if (eb == 4 && g.norm_srk != 0) return false;
     const long long modes = (long long)g.NXH * g.NY;
     if (eb == 8 && zs_vv(g) && modes >= ZS_STREAM_MODES) return true;
-    return modes * g.NZ * 2 * eb >= ZS_STREAM_BYTES && zs_resident_pairs(g, eb) <= ZS_STREAM_PAIRS;
+    const long long bytes = modes * g.NZ * 2 * eb;
+    const int pairs = zs_resident_pairs(g, eb);
+    return (bytes >= ZS_STREAM_BYTES && pairs <= ZS_STREAM_PAIRS) || (eb == 4 && bytes >= ZS_STREAM_BYTES_FEW && pairs <= 3);
 }
 
 // The mixed SRK step keeps the one-sided solve of one thread per mode (k_zsolve_srk): its
@@ -654,10 +658,13 @@ static void zsolve_kp(const ZSolveArgs<T>& a, cudaStream_t s, bool low_only) {
 // Adjacent lanes take the modes (kx, kh), (kx, NY-kh), which share their factors.  Rows are
 // moved R at a time through two register batches, the next batch's loads in flight.  FP64 VV4:
 // R = 2 keeps 5 CTAs of 128 threads per SM, so that the ~74 k modes of a 384 x 384 plane run in
-// one wave (384x384x256: 4 rows 0.318 ms, 3 rows 0.296, 2 rows 0.27-0.29).
+// one wave (384x384x256: 4 rows 0.318 ms, 3 rows 0.296, 2 rows 0.27-0.29).  The others wait for
+// memory with few modes: whole solves in us, VV4 mixed 128x128x2800 1055 with 4 rows, 975 with 6,
+// 791 with 8; HW2 mixed 853 with 6, 781 with 8, 870 with 12; HW2 FP64 256x256x1024 1355 with 4,
+// 1297 with 6, 1291 with 8, and 288x288x700 1263, 1252, 1348.
 template <typename T, bool VV>
 __global__ void __launch_bounds__(128) k_zsolve_stream(ZSolveArgs<T> a) {
-    constexpr int R = sizeof(T) == 8 ? (VV ? 2 : 4) : (VV ? 4 : 6);
+    constexpr int R = sizeof(T) == 8 ? (VV ? 2 : 6) : 8;
     using C = cplx<T>;
     using Q = typename std::conditional<VV, Q4<T>, Q2<T>>::type;
     const Geom& g = a.g;
